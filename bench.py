@@ -504,7 +504,7 @@ def main():
         nsm = torch.cuda.get_device_properties(local_rank).multi_processor_count
         peak = nsm * 128 * sm_mhz * 1e6 / 1e9  # Gop/s
         achieved = ops_launch / (kernel_ms / 1e3) / 1e9
-        kern_name = {1: "level", 2: "sweep"}.get(kern_used, "?")
+        kern_name = {1: "level", 2: "sweep", 3: "diagonal"}.get(kern_used, "?")
         step_lat = sorted(times)
         line = {
             "metric": "CYK/Inside scan Gcells/s", "value": value, "unit": "Gcells/s",

@@ -134,7 +134,7 @@ typedef struct cmgpu_stats {
     int32_t deck_in_smem; /* 1 when the rolling decks live in shared memory */
     int32_t ctas;
     int32_t lanes;        /* work items per CTA                            */
-    int32_t kernel;       /* CMGPU_KERNEL_LEVEL or CMGPU_KERNEL_SWEEP       */
+    int32_t kernel;       /* CMGPU_KERNEL_LEVEL, _SWEEP or _DIAG            */
 } cmgpu_stats;
 
 /* Scan kernels of the QDB scanner (cmgpu_workspace_set_kernel).  Both give
@@ -146,6 +146,7 @@ typedef struct cmgpu_stats {
 #define CMGPU_KERNEL_AUTO 0
 #define CMGPU_KERNEL_LEVEL 1
 #define CMGPU_KERNEL_SWEEP 2
+#define CMGPU_KERNEL_DIAG 3 /* what AUTO runs; reported in the statistics only */
 
 typedef struct cmgpu_model cmgpu_model;
 typedef struct cmgpu_workspace cmgpu_workspace;

@@ -29,6 +29,7 @@
 #include "model_internal.h"
 #include "qdb_kernel.h"
 #include "qdb_plan.h"
+#include "diag_kernel.h"
 #include "sweep_kernel.h"
 
 namespace cmx {
@@ -77,6 +78,8 @@ struct cmgpu_workspace {
     size_t deck_cap = 0;  // elements
     uint32_t *d_sweep = nullptr;  // node-sweep kernel: per-warp decks and BEGL rings
     size_t sweep_cap = 0;         // elements
+    uint32_t *d_diag = nullptr;   // diagonal kernel: one region per CTA
+    size_t diag_cap = 0;          // elements
     // host staging
     Cand *h_cands = nullptr;
     size_t h_cands_cap = 0;
@@ -96,6 +99,7 @@ struct cmgpu_workspace {
         cudaFree(d_counters);
         cudaFree(d_deck);
         cudaFree(d_sweep);
+        cudaFree(d_diag);
         cudaFreeHost(h_cands);
         cudaFreeHost(h_counters);
         if (ev0) cudaEventDestroy(ev0);
@@ -150,6 +154,9 @@ static int get_plan(cmgpu_model *m, int semiring, int qdbidx, DevPlan **out) {
             if ((rc = upload_vec(&dp->sw_bifs, dp->sw.bifs))) return rc;
         }
     }
+    // diagonal plan
+    dp->dg_ok = build_diag_plan(&m->cm.view, p, qdbidx, dp->dg, nullptr);
+    if (dp->dg_ok && (rc = upload_vec(&dp->dg_nodes, dp->dg.nodes))) return rc;
     // per-column work counts by row limit
     const int W = p.W;
     dp->cells_prefix.assign(W + 1, 0.0);
@@ -322,6 +329,8 @@ void report_window(const cmgpu_model *m, int semiring, const Cand *c, size_t n, 
 // ---------------------------------------------------------------------------
 // the batched scan
 // ---------------------------------------------------------------------------
+constexpr int DIAG_WARPS = 8;  // warps per CTA of the diagonal kernel on full batches
+
 struct WinDesc {
     int64_t off;
     int32_t i0, j0;
@@ -412,14 +421,47 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         set_error("node-sweep kernel does not apply to this model: " + dp->sw_why);
         return CMGPU_EINVAL;
     }
-    // AUTO takes the level kernel: measured faster on every workload here
+    // AUTO takes the diagonal kernel wherever it applies (any model with
+    // cm_from_guide's node layout): faster at every size measured, 2.6 against
+    // 26.8 ms for one 300-column window, 112 against 770 ms for 120 uneven
+    // windows.  The level kernel takes the other models.
+    const bool diag = dp->dg_ok && ws->kernel == CMGPU_KERNEL_AUTO;
     const bool sweep = dp->sw_ok && ws->kernel == CMGPU_KERNEL_SWEEP;
     const size_t SMEM_CAP = 227 * 1024 - 1024, SM_CAP = 228 * 1024;
     const int threads = ws->threads;
     int best_c = 0, best_l = 0;
     bool deck_smem = false;
     SweepParams swp{};
-    if (sweep) {
+    DgParams dgp{};
+    if (diag) {
+        dgp.nodes = dp->dg_nodes;
+        dgp.nnodes = (int)dp->dg.nodes.size();
+        dgp.tsc = dp->tsc;
+        dgp.endsc = dp->endsc;
+        dgp.esc = dp->esc;
+        dgp.el_sca = dp->el_sca;
+        dgp.bsv = dp->beginsc_all;
+        dgp.W = pl.W;
+        dgp.ring_cols = dp->dg.ring_cols;
+        dgp.root_dn = pl.root_dn;
+        dgp.root_dxcap = pl.root_dxcap;
+        dgp.inside = sp.inside;
+        dgp.local = sp.local;
+        dgp.begin_key = sp.begin_key;
+        dgp.prefilter = sp.prefilter;
+        dgp.do_null3 = sp.do_null3;
+        for (int a = 0; a < 4; a++) dgp.pf_null[a] = sp.pf_null[a];
+        dgp.pf_omega = sp.pf_omega;
+        dgp.ilog = m->ilog;
+        dgp.ilog_nz = m->ilog_nz;
+        dgp.dsq = d_dsq;
+        dgp.cutoff = cutoff;
+        dgp.region_words = dp->dg.words;
+        // eight warps (256 columns a group) and two CTAs per SM; the shape of
+        // small batches follows their items, below
+        best_l = DIAG_WARPS;
+        best_c = 2;
+    } else if (sweep) {
         // one CTA per SM with as many warps (one work item each) as fit
         const SweepPlan &sw = dp->sw;
         swp.st = dp->sw_st;
@@ -520,11 +562,19 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     // another, and a CTA's time per column grows with its lanes.  Such a
     // batch is cut into about one piece per CTA, and each CTA takes only the
     // few lanes the pieces need (below).
-    const bool small_batch = !sweep && !deck_smem && !plain && ws->chunk <= 0 && ws->lanes <= 0 &&
+    const bool small_batch = !diag && !sweep && !deck_smem && !plain && ws->chunk <= 0 && ws->lanes <= 0 &&
                              total_cols < (int64_t)max_ctas * best_l * 2 * W;
     auto chunk_for = [&](int64_t cols) -> int64_t {
         int64_t chunk = ws->chunk;
-        if (chunk <= 0 && small_batch) {
+        if (chunk <= 0 && diag) {
+            // about four pieces per CTA and none shorter than 4W (the warm-up
+            // costs W/2 columns); with too few columns for that, one piece
+            // per CTA, down to W
+            chunk = std::max<int64_t>((cols + max_ctas - 1) / max_ctas, W);
+            chunk = std::min<int64_t>(chunk, 4 * (int64_t)W);
+            chunk = std::max<int64_t>(chunk, cols / (4 * (int64_t)max_ctas));
+            chunk = std::min<int64_t>(chunk, 32768);
+        } else if (chunk <= 0 && small_batch) {
             chunk = (cols + max_ctas - 1) / max_ctas;
             chunk = std::max<int64_t>(chunk, 2 * (int64_t)W);
             chunk = std::min<int64_t>(chunk, 32768);
@@ -562,8 +612,25 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     ws->stats.work_items = (int64_t)items.size();
     ws->stats.deck_in_smem = deck_smem ? 1 : 0;
     ws->stats.lanes = best_l;
-    ws->stats.kernel = sweep ? CMGPU_KERNEL_SWEEP : CMGPU_KERNEL_LEVEL;
+    ws->stats.kernel = diag ? CMGPU_KERNEL_DIAG : sweep ? CMGPU_KERNEL_SWEEP : CMGPU_KERNEL_LEVEL;
     if (items.empty()) return CMGPU_OK;
+    if (diag) {
+        // no more warps than the longest item has columns; with an SM for
+        // every item, up to sixteen
+        int64_t longest = 0;
+        for (auto &x : items) longest = std::max<int64_t>(longest, (int64_t)x.jend - x.jstart + 1);
+        const int most = (int64_t)items.size() <= ws->sm_count && !plain ? DG_MAX_WARPS : DIAG_WARPS;
+        best_l = (int)std::min<int64_t>(most, (longest + 31) / 32);
+        dgp.ring_len = 1;
+        while (dgp.ring_len < W + 64 * best_l) dgp.ring_len <<= 1;
+        const int occ = diag_occupancy(dgp, best_l);
+        if (occ < 1) {
+            set_error("diagonal kernel cannot be resident");
+            return CMGPU_EDEVICE;
+        }
+        best_c = occ;
+        ws->stats.lanes = best_l;
+    }
 
     if ((rc = ensure_dev(&ws->d_items, &ws->items_cap, items.size()))) return rc;
     CUDA_TRY(cudaMemcpyAsync(ws->d_items, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice,
@@ -573,7 +640,7 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     // well inside it, so the scan is not repeated with a larger buffer.
     const size_t cand_cap = std::max<size_t>({ws->cands_cap, (size_t)1 << 16, (size_t)(total_cols / 4)});
     if ((rc = ensure_dev(&ws->d_cands, &ws->cands_cap, cand_cap))) return rc;
-    if (!sweep && !deck_smem && (int64_t)items.size() < best_l) {
+    if (!diag && !sweep && !deck_smem && (int64_t)items.size() < best_l) {
         // fewer work items than lanes: no deck for lanes that would stay idle
         best_l = (int)items.size();
         sp.lanes = best_l;
@@ -590,7 +657,19 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         }
     }
     int ctas = (int)std::min<int64_t>(((int64_t)items.size() + best_l - 1) / best_l, max_ctas);
-    if (!sweep && !deck_smem) {
+    if (diag) {
+        // the regions stay within half of the free device memory
+        size_t freeb = 0, totalb = 0;
+        CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+        const size_t per_cta = (size_t)dgp.region_words * 4;
+        const size_t have = freeb / 2 + ws->diag_cap * 4;
+        ctas = (int)std::min<int64_t>((int64_t)items.size(), (int64_t)ws->sm_count * best_c);
+        ctas = (int)std::min<size_t>((size_t)ctas, std::max<size_t>(1, have / std::max<size_t>(per_cta, 1)));
+        if ((rc = ensure_dev(&ws->d_diag, &ws->diag_cap, (size_t)dgp.region_words * (size_t)ctas))) return rc;
+        dgp.region = ws->d_diag;
+        dgp.next_item = ws->d_counters;
+        dgp.cand_count = ws->d_counters + 1;
+    } else if (!sweep && !deck_smem) {
         // global decks of large models: keep them within half of the free device memory
         size_t freeb = 0, totalb = 0;
         CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
@@ -606,7 +685,7 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         swp.gmem = ws->d_sweep;
         swp.next_item = ws->d_counters;
         swp.cand_count = ws->d_counters + 1;
-    } else if (!deck_smem) {
+    } else if (!diag && !deck_smem) {
         size_t stride = ((size_t)pl.deck_elems + 31) & ~(size_t)31;
         if ((rc = ensure_dev(&ws->d_deck, &ws->deck_cap, stride * (size_t)ctas * (size_t)best_l))) return rc;
         sp.deck_global = ws->d_deck;
@@ -617,6 +696,14 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
 
     // one launch over items [first, first + n) on `grid` CTAs
     auto launch = [&](size_t first, size_t n, int grid) -> cudaError_t {
+        if (diag) {
+            dgp.items = ws->d_items + first;
+            dgp.nitems = (int)n;
+            dgp.item_base = (int)first;
+            dgp.cands = ws->d_cands;
+            dgp.cand_cap = (int)std::min<size_t>(ws->cands_cap, (size_t)INT32_MAX);
+            return diag_launch(dgp, grid, best_l, ws->stream);
+        }
         if (sweep) {
             swp.items = ws->d_items + first;
             swp.nitems = (int)n;
@@ -642,7 +729,8 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
             for (size_t w = 0; w + 1 < win_first.size(); w++) {
                 size_t f = win_first[w], n = win_first[w + 1] - f;
                 if (n == 0) continue;
-                int grid = (int)std::min<int64_t>(((int64_t)n + best_l - 1) / best_l, max_ctas);
+                int grid = diag ? (int)std::min<int64_t>((int64_t)n, ctas)
+                                : (int)std::min<int64_t>(((int64_t)n + best_l - 1) / best_l, max_ctas);
                 CUDA_TRY(cudaMemsetAsync(ws->d_counters, 0, sizeof(int), ws->stream));
                 CUDA_TRY(launch(f, n, grid));
                 launches++;
@@ -701,10 +789,28 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
             cs[pos[r]++] = x;
         }
     }
+    // The diagonal kernel emits a column's cells in d order but interleaves
+    // the columns: a stable counting sort by column restores (j, d) order.
     auto jd_less = [](const Cand &a, const Cand &b) { return a.j != b.j ? a.j < b.j : a.d < b.d; };
-    for (size_t r = 0; r < items.size(); r++)
-        if (!std::is_sorted(cs.begin() + start[r], cs.begin() + start[r + 1], jd_less))
-            std::sort(cs.begin() + start[r], cs.begin() + start[r + 1], jd_less);
+    auto order_item = [&](size_t r, const WorkItem &it, std::vector<size_t> &at, std::vector<Cand> &tmp) {
+        Cand *f = cs.data() + start[r], *l = cs.data() + start[r + 1];
+        if (std::is_sorted(f, l, jd_less)) return;
+        const size_t ncol = (size_t)(it.jend - it.jreport + 1), n = (size_t)(l - f);
+        if (n > ncol / 8) {
+            at.assign(ncol + 1, 0);
+            for (Cand *x = f; x < l; x++) at[(size_t)(x->j - it.jreport) + 1]++;
+            for (size_t k = 0; k < ncol; k++) at[k + 1] += at[k];
+            tmp.assign(f, l);
+            for (const Cand &x : tmp) f[at[(size_t)(x.j - it.jreport)]++] = x;
+            if (std::is_sorted(f, l, jd_less)) return;
+        }
+        std::sort(f, l, jd_less);
+    };
+    {
+        std::vector<size_t> at;
+        std::vector<Cand> tmp;
+        for (size_t x = 0; x < items.size(); x++) order_item((size_t)rank[x], items[x], at, tmp);
+    }
     if (cells_out) {
         *cells_out = cs;
         return CMGPU_OK;

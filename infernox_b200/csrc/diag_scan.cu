@@ -1,0 +1,726 @@
+// QDB-banded CYK / Inside window scan by diagonals, for sm_100a.
+//
+// Cell (v, j, d) of the scan (generic_scan, src/cm_nohmm.rs:549-763) reads
+// cells of shorter spans (d-1, d-2) at columns j and j-1, and cells of the
+// same span of states below v.  So for one span d every column j is
+// independent, IL's self-loop included (it reads span d-1): a warp takes 32
+// consecutive columns, one per lane, and walks d upwards with no serial chain
+// across lanes and no divergence -- the state type, the band test and the
+// transition scores are the same for all lanes.
+//
+// Order of work.  A work item is a piece of a window; a CTA takes its columns
+// in groups of 32 x warps, left to right.  For a group the nodes run from
+// the last one up, and inside a node d runs from the shortest span stored to
+// the longest.  All states of a node are computed together: its inserts never
+// leave the registers (their left neighbour comes by shuffle), and of the
+// next node only the split states are read, once per span: one load and one
+// store per split cell, instead of one load per child relaxation.
+//   buffers   three node buffers [span][split state][column] used in turn;
+//   BEGL      a ring of W + group columns per bifurcation (a split reads
+//             columns j-k), BEGR the group's columns;
+//   bmax      the ROOT row of local begins (a maximum, so the node order does
+//             not matter);
+//   boundary  the last column of every node is saved for the first column of
+//             the next group, so groups repeat no work.
+// All of it is in a per-CTA region of global memory whose working set (two
+// node buffers, about 0.6 MB at W = 148) stays in L2.
+//
+// Warps run skewed: in phase t warp w runs step t - w of the group's
+// (node, 16 spans) sequence, with one CTA barrier per phase.  So when a warp
+// reads the column left of its first one, the warp on its left has finished
+// those spans; nothing waits on a flag.  Three buffers keep a node's outputs
+// until the warp on the right, one phase behind, has read them.
+//
+// Spans beyond a column's own start (d > j - jstart + 1) and columns past the
+// item's end hold values nobody reads: a valid cell depends on valid cells
+// only.  Rows are addressed by span, residues by a masked ring, so those
+// cells stay in bounds.
+//
+// Measured on one B200 (before: the level kernel of qdb_scan.cu): Inside,
+// non-banded, M = 379, W = 148, 296 windows of 512: 180 Gcells/s; 120 uneven
+// windows 770 -> 112 ms; one window of 300 columns (M = 230) 26.8 -> 2.6 ms;
+// two 1 kb windows of a 4,629-state model, CYK 1,809 -> 63 ms.  Bound: issue
+// and load latency (30% of issue slots at 16 warps per SM); DRAM 17%.
+#include <cuda_runtime.h>
+#include <cstdint>
+#include <type_traits>
+
+#include "devbuf.h"
+#include "diag_kernel.h"
+#include "report_device.cuh"
+#include "cm_internal.h"
+#include "semiring.cuh"
+
+namespace cmx {
+namespace dev {
+
+// Per-warp view of the group it works on.
+struct DgCtx {
+    uint32_t *reg;           // the CTA's region
+    const uint16_t *tbl;     // ILogsum table (shared memory)
+    const uint8_t *ring;     // residues of the item (shared memory)
+    uint32_t *xch;           // [warps][2][DG_CHUNK][2] last column's inserts (shared memory)
+    int nz, rmask;
+    int nw, w, lane, col;    // col = 32 w + lane
+    int jrel;                // column relative to the item's first
+    int ridx;                // jrel modulo the BEGL ring
+    int cj;                  // residue of column j
+    int jmax;                // longest span any lane of the warp can hold (0: no column)
+    int ncols;               // columns of the item
+    int step;                // (node, chunk) steps done, for the exchange slot
+    bool first, last;        // first / last group of the item
+    int item, j, jreport, jend;
+};
+
+__device__ __forceinline__ void dg_phase(int nthreads) {
+    asm volatile("barrier.sync 1, %0;" ::"r"(nthreads) : "memory");
+}
+
+// reduce_c_order (src/cm_nohmm.rs:187-242) of CN child terms and, where the
+// state has a local end, its initial score.  Without one the initial score is
+// -INFTY: combining with it only clamps at -INFTY, which every later
+// combination does anyway, so it is left out (with one child it is not).
+template <class S, int CN>
+__device__ __forceinline__ typename S::T dg_reduce(const typename S::T *t, bool has, typename S::T init,
+                                                   const uint16_t *tb, int nz) {
+    typedef typename S::T T;
+    if constexpr (!S::ORDERED) {
+        T s = has ? init : S::zero();
+#pragma unroll
+        for (int k = 0; k < CN; k++) s = fmaxf(s, t[k]);
+        return s;
+    } else {
+        T s;
+        if constexpr (CN == 1) {
+            s = has ? S::comb(init, t[0], tb, nz) : max(t[0], -INFTY_D);
+            return s;
+        }
+        if constexpr (CN == 2) s = t[1];
+        if constexpr (CN == 3) s = S::comb(t[2], t[1], tb, nz);
+        if constexpr (CN == 4 || CN == 5) s = S::comb(t[CN - 1], t[CN - 2], tb, nz);
+        if constexpr (CN == 6) s = t[5];
+        if (has) s = S::comb(s, init, tb, nz);
+        if constexpr (CN == 4) s = S::comb(s, t[1], tb, nz);
+        if constexpr (CN == 5) {
+            s = S::comb(s, t[1], tb, nz);
+            s = S::comb(s, t[2], tb, nz);
+        }
+        if constexpr (CN == 6) {
+            s = S::comb(s, t[4], tb, nz);
+            s = S::comb(s, t[3], tb, nz);
+            s = S::comb(s, t[2], tb, nz);
+            s = S::comb(s, t[1], tb, nz);
+        }
+        return S::comb(s, t[0], tb, nz);
+    }
+}
+
+// Children in natural order (BEGL_S and ROOT_S, src/cm_nohmm.rs:601-611, :700-719).
+template <class S, int CN>
+__device__ __forceinline__ typename S::T dg_natural(const typename S::T *t, bool has, typename S::T init,
+                                                    const uint16_t *tb, int nz) {
+    typedef typename S::T T;
+    if constexpr (!S::ORDERED) {
+        return dg_reduce<S, CN>(t, has, init, tb, nz);
+    } else {
+        T s = has ? S::comb(init, t[0], tb, nz) : max(t[0], -INFTY_D);
+#pragma unroll
+        for (int k = 1; k < CN; k++) s = S::comb(s, t[k], tb, nz);
+        return s;
+    }
+}
+
+// Local begins: the larger of two ROOT values as begin_less orders them
+// (with begin_key, -INFTY is held as INT_MIN).
+template <class S>
+__device__ __forceinline__ typename S::T dg_begin_max(typename S::T a, typename S::T c) {
+    return a < c ? c : a;
+}
+template <class S>
+__device__ __forceinline__ typename S::T dg_begin_key(int key, typename S::T c) {
+    if constexpr (S::ORDERED)
+        if (key && c == -INFTY_D) return INT32_MIN;
+    return c;
+}
+template <class S>
+__device__ __forceinline__ typename S::T dg_begin_none(int key) {
+    if constexpr (S::ORDERED) return key ? INT32_MIN : -INFTY_D;
+    else return -INFINITY;
+}
+
+// One node over the group's columns: NT its type, NN the split states of the
+// next node.
+//
+// Two versions of the same step: `edge` tests every band and row range;
+// `inner` runs where nothing needs a test (every state in band, the child
+// rows stored, no d = 0) and at most the first state has a local begin or a
+// local end, which is how local models are configured.  Child values are
+// loaded two spans ahead, so their latency is covered by two steps.
+template <class S, int NT, int NN>
+__device__ __forceinline__ void dg_node(const DgParams &p, DgCtx &c, const DgNode *np) {
+    typedef typename S::T T;
+    constexpr bool HAS_IL = NT == MATP_ND || NT == MATL_ND || NT == ROOT_ND || NT == BEGR_ND;
+    constexpr bool HAS_IR = NT == MATP_ND || NT == MATR_ND || NT == ROOT_ND;
+    constexpr bool LEFT = HAS_IR;  // MP, MR and IR read column j-1
+    constexpr int NSPLIT = NT == MATP_ND ? 4 : (NT == MATL_ND || NT == MATR_ND) ? 2 : 1;
+    constexpr int QIL = NSPLIT, QIR = HAS_IL ? NSPLIT + 1 : NSPLIT;  // insert states within the node
+    constexpr int NI = (HAS_IL ? 1 : 0) + (HAS_IR ? 1 : 0);
+    constexpr int CN = NI + NN;  // children of a split state
+    constexpr int MP = NT == MATP_ND ? 0 : -1, ML = NT == MATP_ND ? 1 : NT == MATL_ND ? 0 : -1,
+                  MR = NT == MATP_ND ? 2 : NT == MATR_ND ? 0 : -1;
+    const unsigned FULL = 0xffffffffu;
+    const T ZERO = S::zero();
+    const int v0 = np->v0, rlo = np->rlo, clo = np->clo, chi = np->chi;
+    const int rhi = min(np->rhi, c.ncols);  // no column of the item holds a longer span
+    const bool cend = np->next_end != 0;
+    const T cinit = S::ld(&np->cinit0);
+    const int endmask = np->endmask, beginmask = np->beginmask;
+    const bool need_left = np->need_left != 0;
+    uint32_t *out = c.reg + np->out_off;
+    int ostride;
+    if (NT == BEGL_ND) {
+        out += c.ridx;
+        ostride = p.ring_cols;
+    } else if (NT == BEGR_ND) {
+        out += c.col;
+        ostride = DG_COLS;
+    } else {
+        out += 32 + c.col;
+        ostride = DG_ROW;
+    }
+    const uint32_t *in = c.reg + np->in_off + 32 + c.col;
+    uint32_t *bnd = c.reg + np->bnd_off;
+    uint32_t *bndi = bnd + (int64_t)(np->rhi - rlo + 1) * DG_SLOTS;
+    T *const bmax = reinterpret_cast<T *>(c.reg + c.col);
+
+    // spans the inner step takes
+    int ilo = max(1, p.root_dn), ihi = min(rhi, p.root_dxcap);
+#pragma unroll
+    for (int q = 0; q < NSPLIT + NI; q++) {
+        ilo = max(ilo, (int)np->dn[q]);
+        ihi = min(ihi, (int)np->dx[q]);
+    }
+    ilo = max(ilo, clo - 1);
+    ihi = min(ihi, chi - 2);
+    if (cend || ((endmask | beginmask) & ~1)) ihi = -1;
+    const bool end0 = (endmask & 1) != 0, beg0 = p.local && (beginmask & 1) != 0;
+    const T es0 = end0 ? S::ldg(p.endsc + v0) : ZERO;
+    const T bs0 = beg0 ? S::ldg(p.bsv + v0) : ZERO;
+
+    // transition scores, in registers
+    T ts[NSPLIT][CN], til[HAS_IL ? CN : 1], tir[HAS_IR ? NN + 1 : 1];
+#pragma unroll
+    for (int q = 0; q < NSPLIT; q++)
+#pragma unroll
+        for (int k = 0; k < CN; k++) ts[q][k] = S::ldg(p.tsc + (v0 + q) * 6 + k);
+    if constexpr (HAS_IL)
+#pragma unroll
+        for (int k = 0; k < CN; k++) til[k] = S::ldg(p.tsc + (v0 + QIL) * 6 + k);
+    if constexpr (HAS_IR)
+#pragma unroll
+        for (int k = 0; k < NN + 1; k++) tir[k] = S::ldg(p.tsc + (v0 + QIR) * 6 + k);
+
+    auto ldx = [&](int y, int d, int shift) -> T {  // split state y of the next node at (j - shift, d)
+        if (cend) return d == 0 ? cinit : ZERO;
+        if (d < clo || d > chi) return ZERO;
+        return S::ld(in + (int64_t)(d - clo) * DG_ROW + y * DG_PITCH - shift);
+    };
+    const uint32_t *esc0 = p.esc + (int64_t)v0 * ESC;
+    const uint32_t *escr = esc0 + c.cj;
+
+    // xp, xc, xc1: column j at d-1, d, d+1; xl2, xl1, xl0: column j-1 at
+    // d-2, d-1, d; il*, ir*: the inserts at d-1 (and column j-1, d-1 and d-2)
+    T xp[NN], xc[NN], xc1[NN], xl2[NN], xl1[NN], xl0[NN];
+    T ilp = ZERO, irp = ZERO, il1 = ZERO, il2 = ZERO, ir1 = ZERO, ir2 = ZERO;
+    int d = rlo;
+#pragma unroll
+    for (int y = 0; y < NN; y++) {
+        xp[y] = ldx(y, d - 1, 0);
+        xc[y] = ldx(y, d, 0);
+        xc1[y] = ldx(y, d + 1, 0);
+        if (LEFT) {
+            xl2[y] = ldx(y, d - 2, 1);
+            xl1[y] = ldx(y, d - 1, 1);
+            xl0[y] = ldx(y, d, 1);
+        }
+    }
+    int ci = HAS_IL ? c.ring[(c.jrel - d + 1) & c.rmask] : 0;  // residue j-d+1
+    const int nthreads = c.nw * 32;
+    for (int r0 = rlo; r0 <= rhi; r0 += DG_CHUNK) {
+        const int rend = min(r0 + DG_CHUNK - 1, rhi);
+        const int dstop = min(rend, c.jmax);
+        const int slot = c.step & 1;
+        // the inserts of the column left of the warp: lane r holds span r0 + r
+        T hil = ZERO, hir = ZERO;
+        if constexpr (HAS_IR) {
+            const int r = c.lane & (DG_CHUNK - 1);
+            if (c.w > 0) {
+                const uint32_t *lp = c.xch + (((c.w - 1) * 2 + slot) * DG_CHUNK + r) * 2;
+                hil = S::ld(lp);
+                hir = S::ld(lp + 1);
+            } else if (!c.first && r0 + r <= rend) {
+                const uint32_t *lp = bndi + (int64_t)(r0 + r - rlo) * 2;
+                hil = S::ld(lp);
+                hir = S::ld(lp + 1);
+            }
+        }
+        uint32_t *xs = c.xch + (c.w * 2 + slot) * (DG_CHUNK * 2);
+        // the column left of the group (its parent reads it)
+        if (NT != ROOT_ND && need_left && c.w == 0) {
+            const int r = c.lane & (DG_CHUNK - 1), h = r0 + r;
+            if (c.lane < DG_CHUNK && h <= dstop) {
+#pragma unroll
+                for (int q = 0; q < NSPLIT; q++) {
+                    T x = h == 0 ? S::ld(&np->init0[q]) : ZERO;
+                    if (!c.first) x = S::ld(bnd + (h - rlo) * DG_SLOTS + q);
+                    S::st(out - c.lane + (int64_t)(h - rlo) * DG_ROW + q * DG_PITCH - 1, x);
+                }
+            }
+        }
+
+        // one span; px, po: rows d of the child (column j) and of the outputs
+        auto step = [&](auto inner_c, const uint32_t *px, uint32_t *po, T &bm) {
+            constexpr bool INNER = decltype(inner_c)::value;
+            T xn[NN], xln[NN];
+#pragma unroll
+            for (int y = 0; y < NN; y++) {
+                xn[y] = INNER ? S::ld(px + 2 * DG_ROW + y * DG_PITCH) : ldx(y, d + 2, 0);
+                if (LEFT) xln[y] = INNER ? S::ld(px + DG_ROW + y * DG_PITCH - 1) : ldx(y, d + 1, 1);
+            }
+            const uint32_t *esci = esc0 + ci;
+            T eil, eml, emp;
+            if (HAS_IL) eil = S::ldg(esci + QIL * ESC);
+            if (ML >= 0) eml = S::ldg(esci + (ML < 0 ? 0 : ML) * ESC);
+            if (MP >= 0) emp = S::ldg(escr + ci * KP);
+            if (HAS_IL) ci = c.ring[(c.jrel - d) & c.rmask];
+            T bmn = ZERO;
+            if (INNER && beg0) bmn = bmax[(int64_t)(d + 1) * DG_COLS];  // d + 1 <= W
+            const T el0 = INNER && (NT != BEGL_ND && NT != BEGR_ND) ? ZERO : S::ldg(p.el_sca + d);
+            const T el1 = INNER && NT == MATP_ND ? ZERO : S::ldg(p.el_sca + max(d - 1, 0));
+            const T el2 = NT == MATP_ND ? S::ldg(p.el_sca + max(d - 2, 0)) : ZERO;
+            T bc = dg_begin_none<S>(p.begin_key);
+            auto begin = [&](int q, T x) {
+                if (!INNER && (beginmask >> q & 1))
+                    bc = dg_begin_max<S>(bc, dg_begin_key<S>(p.begin_key, S::add(x, S::ldg(p.bsv + v0 + q))));
+            };
+            auto in_band = [&](int q) { return INNER || (d >= np->dn[q] && d <= np->dx[q]); };
+            auto fill = [&](int q) -> T { return !INNER && d == 0 ? S::ld(&np->init0[q]) : ZERO; };
+            auto has = [&](int q) { return INNER ? (q == 0 && end0) : (endmask >> q & 1) != 0; };
+            auto init = [&](int q, T el) -> T {
+                return INNER ? S::add(el, es0) : S::add(el, S::ldg(p.endsc + v0 + q));
+            };
+            T iln = ZERO, irn = ZERO;
+            T val[NSPLIT];
+            // inserts
+            if constexpr (HAS_IL) {
+                iln = fill(QIL);
+                if (in_band(QIL)) {
+                    T t[CN];
+                    t[0] = S::add(ilp, til[0]);
+                    if (HAS_IR) t[1] = S::add(irp, til[1]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[NI + y] = S::add(xp[y], til[NI + y]);
+                    iln = dg_reduce<S, CN>(t, has(QIL), INNER ? ZERO : init(QIL, el1), c.tbl, c.nz);
+                    iln = S::add(iln, eil);
+                    begin(QIL, iln);
+                }
+            }
+            if constexpr (HAS_IR) {
+                irn = fill(QIR);
+                if (in_band(QIR)) {
+                    T t[NN + 1];
+                    t[0] = S::add(ir1, tir[0]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[1 + y] = S::add(xl1[y], tir[1 + y]);
+                    irn = dg_reduce<S, NN + 1>(t, has(QIR), INNER ? ZERO : init(QIR, el1), c.tbl, c.nz);
+                    irn = S::add(irn, S::ldg(escr + QIR * ESC));
+                    begin(QIR, irn);
+                }
+            }
+            // split states
+#pragma unroll
+            for (int q = 0; q < NSPLIT; q++) {
+                val[q] = fill(q);
+                if (!in_band(q)) continue;
+                T t[CN];
+                T x;
+                if (q == MP) {
+                    t[0] = S::add(il2, ts[q][0]);
+                    t[1] = S::add(ir2, ts[q][1]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[NI + y] = S::add(xl2[y], ts[q][NI + y]);
+                    x = S::add(dg_reduce<S, CN>(t, has(q), init(q, el2), c.tbl, c.nz), emp);
+                } else if (q == ML) {
+                    t[0] = S::add(ilp, ts[q][0]);
+                    if (HAS_IR) t[1] = S::add(irp, ts[q][1]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[NI + y] = S::add(xp[y], ts[q][NI + y]);
+                    x = S::add(dg_reduce<S, CN>(t, has(q), init(q, el1), c.tbl, c.nz), eml);
+                } else if (q == MR) {
+                    t[0] = S::add(HAS_IL ? il1 : ir1, ts[q][0]);
+                    if (HAS_IL) t[1] = S::add(ir1, ts[q][1]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[NI + y] = S::add(xl1[y], ts[q][NI + y]);
+                    x = dg_reduce<S, CN>(t, has(q), init(q, el1), c.tbl, c.nz);
+                    x = S::add(x, S::ldg(escr + q * ESC));
+                } else {  // D, S
+                    if (HAS_IL) t[0] = S::add(iln, ts[q][0]);
+                    if (HAS_IR) t[HAS_IL ? 1 : 0] = S::add(irn, ts[q][HAS_IL ? 1 : 0]);
+#pragma unroll
+                    for (int y = 0; y < NN; y++) t[NI + y] = S::add(xc[y], ts[q][NI + y]);
+                    if (NT == ROOT_ND) x = dg_natural<S, CN>(t, false, ZERO, c.tbl, c.nz);
+                    else if (NT == BEGL_ND) x = dg_natural<S, CN>(t, has(q), init(q, el0), c.tbl, c.nz);
+                    else x = dg_reduce<S, CN>(t, has(q), init(q, el0), c.tbl, c.nz);
+                }
+                val[q] = x;
+                if (NT != ROOT_ND) begin(q, x);
+            }
+            if (NT != ROOT_ND)
+#pragma unroll
+                for (int q = 0; q < NSPLIT; q++) S::st(po + q * DG_PITCH, val[q]);
+            if (INNER) {
+                if (beg0) {
+                    bmax[(int64_t)d * DG_COLS] =
+                        dg_begin_max<S>(bm, dg_begin_key<S>(p.begin_key, S::add(val[0], bs0)));
+                    bm = bmn;
+                }
+            } else if (d >= p.root_dn && d <= p.root_dxcap) {
+                T *bp = bmax + (int64_t)d * DG_COLS;
+                if (p.local && beginmask) *bp = dg_begin_max<S>(*bp, bc);
+                if (NT == ROOT_ND) {
+                    T a = val[0];
+                    if (p.local && dg_begin_key<S>(p.begin_key, a) < *bp) a = *bp;
+                    if (p.prefilter) {
+                        *bp = a;
+                    } else {
+                        const float sc = S::bits(a);
+                        const bool hit = sc >= p.cutoff && sc > IMPOSSIBLE_D + 1.0f && d <= c.jrel + 1 &&
+                                         c.j >= c.jreport && c.j <= c.jend;
+                        emit_cand(p, c.lane, hit, c.item, c.j, d, S::u(a));
+                    }
+                }
+            }
+            // hand the inserts to the column on the right
+            if constexpr (HAS_IR) {
+                T li = ZERO, lr, t;
+                if (HAS_IL) {
+                    li = __shfl_up_sync(FULL, iln, 1);
+                    t = __shfl_sync(FULL, hil, d - r0);
+                    if (c.lane == 0) li = t;
+                }
+                lr = __shfl_up_sync(FULL, irn, 1);
+                t = __shfl_sync(FULL, hir, d - r0);
+                if (c.lane == 0) lr = t;
+                if (c.lane == 31) {
+                    if (HAS_IL) S::st(xs + (d - r0) * 2, iln);
+                    S::st(xs + (d - r0) * 2 + 1, irn);
+                }
+                il2 = il1;
+                il1 = li;
+                ir2 = ir1;
+                ir1 = lr;
+            }
+            ilp = iln;
+            irp = irn;
+#pragma unroll
+            for (int y = 0; y < NN; y++) {
+                xp[y] = xc[y];
+                xc[y] = xc1[y];
+                xc1[y] = xn[y];
+                if (LEFT) {
+                    xl2[y] = xl1[y];
+                    xl1[y] = xl0[y];
+                    xl0[y] = xln[y];
+                }
+            }
+        };
+        while (d <= dstop) {
+            T bm = ZERO;
+            uint32_t *po = out + (int64_t)(d - rlo) * ostride;
+            const int iend = min(dstop, ihi);
+            if (NT != ROOT_ND && d >= ilo && d <= iend) {
+                const uint32_t *px = in + (int64_t)(d - clo) * DG_ROW;
+                if (beg0) bm = bmax[(int64_t)d * DG_COLS];
+#pragma unroll 2
+                for (; d <= iend; d++) {
+                    step(std::true_type(), px, po, bm);
+                    px += DG_ROW;
+                    po += ostride;
+                }
+            } else {
+                step(std::false_type(), nullptr, po, bm);
+                d++;
+            }
+        }
+        // the group's last column, for the next group
+        if (!c.last && c.w == c.nw - 1) {
+            __syncwarp();
+            const int r = c.lane & (DG_CHUNK - 1), h = r0 + r;
+            if (c.lane < DG_CHUNK && h <= dstop) {
+                if (NT != ROOT_ND && need_left)
+#pragma unroll
+                    for (int q = 0; q < NSPLIT; q++)
+                        S::st(bnd + (h - rlo) * DG_SLOTS + q,
+                              S::ld(out + (31 - c.lane) + (int64_t)(h - rlo) * DG_ROW + q * DG_PITCH));
+                if (HAS_IR) {
+                    bndi[(int64_t)(h - rlo) * 2] = xs[r * 2];
+                    bndi[(int64_t)(h - rlo) * 2 + 1] = xs[r * 2 + 1];
+                }
+            }
+        }
+        c.step++;
+        dg_phase(nthreads);
+    }
+}
+
+// Bifurcation node: alpha[v][d] = init (+) over k ascending of
+// BEGL(j-k, d-k) + BEGR(j, k) (src/cm_nohmm.rs:578-600).  Four spans at a
+// time share the BEGR loads and give four independent chains.
+template <class S>
+__device__ __forceinline__ void dg_bif(const DgParams &p, DgCtx &c, const DgNode *np) {
+    typedef typename S::T T;
+    const T ZERO = S::zero();
+    const int v0 = np->v0, rlo = np->rlo, rhi = min(np->rhi, c.ncols), nthreads = c.nw * 32;
+    const int dn = np->dn[0], dx = np->dx[0];
+    const int kdn_y = np->kdn_y, kdx_y = np->kdx_y, kdn_w = np->kdn_w, kdx_w = np->kdx_w;
+    const uint32_t *begl = c.reg + np->begl_off, *begr = c.reg + np->begr_off + c.col;
+    const int llo = np->begl_lo, ylo = np->begr_lo, RC = p.ring_cols;
+    const T linit = S::ld(&np->begl_init0);
+    const bool need_left = np->need_left != 0, has = (np->endmask & 1) != 0, beg = (np->beginmask & 1) != 0;
+    const T bs = beg ? S::ldg(p.bsv + v0) : ZERO, es = has ? S::ldg(p.endsc + v0) : ZERO;
+    uint32_t *out = c.reg + np->out_off + 32 + c.col;
+    uint32_t *bnd = c.reg + np->bnd_off;
+    constexpr int U = 4;
+    for (int r0 = rlo; r0 <= rhi; r0 += DG_CHUNK) {
+        const int dstop = min(min(r0 + DG_CHUNK - 1, rhi), c.jmax);
+        for (int d0 = r0; d0 <= dstop; d0 += U) {
+            T acc[U];
+            int klo[U], khi[U];
+            int ka = 1 << 30, kb = -1, ba = 0, bb = 1 << 30;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int d = d0 + u;
+                acc[u] = has ? S::add(S::ldg(p.el_sca + min(d, p.W)), es) : ZERO;
+                klo[u] = max(0, max(kdn_y, d - kdx_w));
+                khi[u] = min(kdx_y, d - kdn_w);
+                if (d < dn || d > dx || d > dstop) klo[u] = 0, khi[u] = -1;
+                if (khi[u] >= klo[u]) {
+                    ka = min(ka, klo[u]);
+                    kb = max(kb, khi[u]);
+                }
+                // splits every span has, with a BEGL span of at least 1
+                ba = max(ba, klo[u]);
+                bb = min(bb, min(khi[u], d - 1));
+            }
+            auto ring = [&](int k) {
+                int x = c.ridx - k;
+                return x < 0 ? x + RC : x;
+            };
+            auto edge = [&](int k0, int k1) {
+                for (int k = k0; k <= k1; k++) {
+                    const T rv = S::ld(begr + (int64_t)(k - ylo) * DG_COLS);
+                    const uint32_t *lc = begl + ring(k) + (int64_t)(d0 - k - llo) * RC;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (k < klo[u] || k > khi[u]) continue;
+                        const T lv = k == d0 + u ? linit : S::ld(lc + (int64_t)u * RC);
+                        acc[u] = S::ORDERED ? S::comb(acc[u], S::add(lv, rv), c.tbl, c.nz)
+                                            : (T)fmaxf((float)acc[u], (float)S::add(lv, rv));
+                    }
+                }
+            };
+            if (bb < ba) {
+                edge(ka, kb);
+            } else {
+                edge(ka, ba - 1);
+                const uint32_t *rp = begr + (int64_t)(ba - ylo) * DG_COLS;
+                int rx = ring(ba);
+                const uint32_t *lr = begl + (int64_t)(d0 - ba - llo) * RC;
+#pragma unroll 4
+                for (int k = ba; k <= bb; k++) {
+                    const T rv = S::ld(rp);
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const T x = S::add(S::ld(lr + rx + (int64_t)u * RC), rv);
+                        if constexpr (S::ORDERED) acc[u] = S::comb(acc[u], x, c.tbl, c.nz);
+                        else acc[u] = fmaxf(acc[u], x);
+                    }
+                    rp += DG_COLS;
+                    lr -= RC;
+                    rx = rx == 0 ? RC - 1 : rx - 1;
+                }
+                edge(bb + 1, kb);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int d = d0 + u;
+                if (d > dstop) continue;
+                const bool in = d >= dn && d <= dx;
+                const T fill = d == 0 ? S::ld(&np->init0[0]) : ZERO;
+                const T x = in ? acc[u] : fill;
+                uint32_t *o = out + (int64_t)(d - rlo) * DG_ROW;
+                S::st(o, x);
+                if (need_left) {
+                    // the column left of the group, and the group's last one
+                    if (c.w == 0 && c.lane == 0) S::st(o - 1, c.first ? fill : S::ld(bnd + (d - rlo) * DG_SLOTS));
+                    if (!c.last && c.w == c.nw - 1 && c.lane == 31) S::st(bnd + (d - rlo) * DG_SLOTS, x);
+                }
+                if (p.local && beg && in && d >= p.root_dn && d <= p.root_dxcap) {
+                    T *bm = reinterpret_cast<T *>(c.reg + c.col + (int64_t)d * DG_COLS);
+                    *bm = dg_begin_max<S>(*bm, dg_begin_key<S>(p.begin_key, S::add(x, bs)));
+                }
+            }
+        }
+        c.step++;
+        dg_phase(nthreads);
+    }
+}
+
+// Report pre-filter of the warp's columns, one column per lane (the rule of
+// prefilter_row in qdb_scan.cu: with approximate corrected scores, a cell is
+// dropped only when it surely can neither be reported nor raise the running
+// maximum of the reported scores).  null3 only lowers a score, so a cell
+// whose uncorrected score is already below the running maximum needs none.
+template <class S>
+__device__ void dg_prefilter(const DgParams &p, const DgCtx &c) {
+    const uint32_t *row = c.reg + c.col;
+    uint32_t c01 = 0, c23 = 0;  // counts of residues 0,1 / 2,3 in j-d+1..j, 16 bits each
+    float run = -INFINITY;
+    const bool live = c.j >= c.jreport && c.j <= c.jend;
+    const int dmax = min(p.root_dxcap, c.jmax);
+    for (int d = 1; d <= dmax; d++) {
+        const int r = c.ring[(c.jrel - d + 1) & c.rmask];
+        c01 += (r == 0 ? 1u : 0u) | (r == 1 ? 0x10000u : 0u);
+        c23 += (r == 2 ? 1u : 0u) | (r == 3 ? 0x10000u : 0u);
+        bool hit = false;
+        uint32_t raw = 0;
+        if (live && d >= p.root_dn && d <= c.jrel + 1) {
+            raw = row[(int64_t)d * DG_COLS];
+            const float bits = S::bits(S::ld(row + (int64_t)d * DG_COLS));
+            const float bar = run == -INFINITY ? -INFINITY : run - pf_margin(run);
+            if (bits > IMPOSSIBLE_D + 1.0f && !(bits + pf_margin(bits) <= bar)) {
+                float x = bits;
+                if (p.do_null3) {
+                    const uint32_t n[4] = {c01 & 0xffffu, c01 >> 16, c23 & 0xffffu, c23 >> 16};
+                    x = __fsub_rn(x, null3_approx(p, n, d));
+                }
+                const float m = pf_margin(x);
+                hit = x + m >= p.cutoff && (run == -INFINITY || x + m > bar);
+                if (x - m >= p.cutoff) run = fmaxf(run, x);
+            }
+        }
+        emit_cand(p, c.lane, hit, c.item, c.j, d, raw);
+    }
+}
+
+template <bool INS>
+__global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid_constant__ DgParams p) {
+    typedef Sem<INS> S;
+    typedef typename S::T T;
+    extern __shared__ __align__(16) uint32_t dg_smem[];
+    __shared__ int s_item;
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    DgCtx c;
+    c.nw = nthreads >> 5;
+    c.w = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform over the warp
+    c.lane = tid & 31;
+    c.col = tid;
+    c.reg = p.region + (int64_t)blockIdx.x * p.region_words;
+    c.xch = dg_smem;
+    uint8_t *ring = reinterpret_cast<uint8_t *>(dg_smem + c.nw * 2 * DG_CHUNK * 2);
+    uint16_t *tbl = reinterpret_cast<uint16_t *>(ring + p.ring_len);
+    c.ring = ring;
+    c.tbl = tbl;
+    c.nz = p.ilog_nz;
+    c.rmask = p.ring_len - 1;
+    if (INS)
+        for (int x = tid; x <= p.ilog_nz; x += nthreads) tbl[x] = p.ilog[x];
+    for (int x = tid; x < p.ring_len; x += nthreads) ring[x] = 0;
+    const T NONE = dg_begin_none<S>(p.begin_key);
+    const int cols = c.nw * 32;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(p.next_item, 1);
+        __syncthreads();
+        const int it = s_item;
+        if (it >= p.nitems) break;
+        const WorkItem wi = p.items[it];
+        c.item = p.item_base + it;
+        c.jreport = wi.jreport;
+        c.jend = wi.jend;
+        c.ncols = wi.jend - wi.jstart + 1;
+        const uint8_t *dsq = p.dsq + wi.dsq_off;
+        c.step = 0;
+        for (int x = 0; x < c.w; x++) dg_phase(nthreads);
+        for (int g0 = 0; g0 < c.ncols; g0 += cols) {
+            c.first = g0 == 0;
+            c.last = g0 + cols >= c.ncols;
+            c.jrel = g0 + c.col;
+            c.j = wi.jstart + c.jrel;
+            c.ridx = c.jrel % p.ring_cols;
+            const int w0 = g0 + c.w * 32;  // the warp's first column
+            c.jmax = w0 < c.ncols ? min(p.W, min(w0 + 32, c.ncols)) : 0;
+            int r = c.j <= wi.jend ? __ldg(dsq + c.j) : 0;
+            r = r > 17 ? 17 : r;
+            ring[c.jrel & c.rmask] = (uint8_t)r;
+            c.cj = r;
+            __syncwarp();
+            if (p.local && c.jmax > 0)
+                for (int d = p.root_dn; d <= min(p.root_dxcap, c.jmax); d++)
+                    S::st(c.reg + c.col + (int64_t)d * DG_COLS, NONE);
+            for (int n = 0; n < p.nnodes; n++) {
+                const DgNode *np = p.nodes + n;
+                switch (np->type * 8 + np->nn) {
+                case MATP_ND * 8 + 1: dg_node<S, MATP_ND, 1>(p, c, np); break;
+                case MATP_ND * 8 + 2: dg_node<S, MATP_ND, 2>(p, c, np); break;
+                case MATP_ND * 8 + 4: dg_node<S, MATP_ND, 4>(p, c, np); break;
+                case MATL_ND * 8 + 1: dg_node<S, MATL_ND, 1>(p, c, np); break;
+                case MATL_ND * 8 + 2: dg_node<S, MATL_ND, 2>(p, c, np); break;
+                case MATL_ND * 8 + 4: dg_node<S, MATL_ND, 4>(p, c, np); break;
+                case MATR_ND * 8 + 1: dg_node<S, MATR_ND, 1>(p, c, np); break;
+                case MATR_ND * 8 + 2: dg_node<S, MATR_ND, 2>(p, c, np); break;
+                case MATR_ND * 8 + 4: dg_node<S, MATR_ND, 4>(p, c, np); break;
+                case BEGL_ND * 8 + 1: dg_node<S, BEGL_ND, 1>(p, c, np); break;
+                case BEGL_ND * 8 + 2: dg_node<S, BEGL_ND, 2>(p, c, np); break;
+                case BEGL_ND * 8 + 4: dg_node<S, BEGL_ND, 4>(p, c, np); break;
+                case BEGR_ND * 8 + 1: dg_node<S, BEGR_ND, 1>(p, c, np); break;
+                case BEGR_ND * 8 + 2: dg_node<S, BEGR_ND, 2>(p, c, np); break;
+                case BEGR_ND * 8 + 4: dg_node<S, BEGR_ND, 4>(p, c, np); break;
+                case ROOT_ND * 8 + 1: dg_node<S, ROOT_ND, 1>(p, c, np); break;
+                case ROOT_ND * 8 + 2: dg_node<S, ROOT_ND, 2>(p, c, np); break;
+                case ROOT_ND * 8 + 4: dg_node<S, ROOT_ND, 4>(p, c, np); break;
+                default: dg_bif<S>(p, c, np); break;
+                }
+            }
+            if (p.prefilter && c.jmax > 0) dg_prefilter<S>(p, c);
+        }
+        for (int x = c.w; x < c.nw - 1; x++) dg_phase(nthreads);
+        __syncthreads();
+    }
+}
+
+static size_t dg_smem_bytes(const DgParams &p, int warps) {
+    size_t b = (size_t)warps * 2 * DG_CHUNK * 2 * 4 + (size_t)p.ring_len;
+    if (p.inside) b += ((size_t)(p.ilog_nz + 1) * 2 + 15) & ~(size_t)15;
+    return b;
+}
+
+}  // namespace dev
+
+int diag_occupancy(const DgParams &p, int warps) {
+    int n = 0;
+    const size_t smem = dev::dg_smem_bytes(p, warps);
+    auto k = p.inside ? dev::diag_kernel<true> : dev::diag_kernel<false>;
+    if (allow_max_dynamic_smem(k) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, warps * 32, smem) != cudaSuccess) return 0;
+    return n;
+}
+
+cudaError_t diag_launch(const DgParams &p, int ctas, int warps, cudaStream_t s) {
+    auto k = p.inside ? dev::diag_kernel<true> : dev::diag_kernel<false>;
+    cudaError_t e = allow_max_dynamic_smem(k);
+    if (e != cudaSuccess) return e;
+    k<<<ctas, warps * 32, dev::dg_smem_bytes(p, warps), s>>>(p);
+    return cudaGetLastError();
+}
+
+}  // namespace cmx

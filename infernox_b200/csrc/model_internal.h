@@ -12,6 +12,7 @@
 
 #include "../../include/cmscan_gpu.h"
 #include "cm_internal.h"
+#include "diag_kernel.h"
 #include "qdb_kernel.h"
 #include "qdb_plan.h"
 #include "sweep_plan.h"
@@ -113,7 +114,12 @@ struct DevPlan {
     SwIO *sw_io = nullptr;
     SwBif *sw_bifs = nullptr;
     uint32_t *init0 = nullptr;
+    // diagonal kernel (diag_scan.cu); dg_ok false when the model is outside its scope
+    bool dg_ok = false;
+    DiagPlan dg;
+    DgNode *dg_nodes = nullptr;
     ~DevPlan() {
+        cudaFree(dg_nodes);
         cudaFree(sw_st);
         cudaFree(sw_kid);
         cudaFree(sw_nodes);

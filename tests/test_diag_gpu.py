@@ -1,0 +1,71 @@
+"""The diagonal scan kernel (what KERNEL_AUTO runs) at the sizes where its
+tiling can go wrong: a warp's 32 columns, a CTA's group of columns, the last
+partial group, windows shorter than W, forced pieces -- against the oracle
+bit for bit, and every ROOT cell against the level kernel over all semirings,
+band sets and configurations."""
+import numpy as np
+import pytest
+
+import oracle
+from infernox_b200 import _native as N
+from infernox_b200 import scan
+from infernox_b200.scan import CYK_F32, INSIDE_I32, KERNEL_LEVEL, NOQDB, QDB1, QDB2
+
+from helpers import frame, models, oracle_cfg, planted_seq
+
+pytestmark = pytest.mark.gpu
+
+DIAG = 3  # CMGPU_KERNEL_DIAG in the statistics
+
+
+def seq_of(cm, n, seed):
+    if n < 100:
+        return np.random.default_rng(seed).integers(0, 4, n).astype(np.uint8)
+    return planted_seq(cm, n, 0.5, 1 + n // 1000, seed=seed, degenerate=0.01)
+
+
+def bits(hits):
+    return [(h[0], h[1], np.float32(h[2]).tobytes(), np.float32(h[3]).tobytes()) for h in hits]
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 256, 257, 511, 512, 513, 1100])
+@pytest.mark.parametrize("name", ["small0", "mb3"])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, QDB2), (INSIDE_I32, NOQDB)])
+def test_edges_match_oracle(name, n, sr, band):
+    cm, _, l = models(name)
+    dsq = frame(seq_of(cm, n, 100 + n))
+    ref, _, _, _ = oracle.qdb_scan(oracle_cfg(name, True), sr, band, dsq, 1, n, -20.0, True)
+    s = scan.Scanner(l)
+    got = s.generic_scan(sr, band, dsq, 1, n, -20.0, True)
+    assert s.stats()["kernel"] == DIAG
+    assert bits(got) == bits(ref)
+
+
+@pytest.mark.parametrize("name", ["small0", "trna", "small2", "mb3", "cfg2"])
+@pytest.mark.parametrize("local", [False, True])
+@pytest.mark.parametrize("sr", [CYK_F32, INSIDE_I32])
+@pytest.mark.parametrize("band", [NOQDB, QDB1, QDB2])
+def test_every_root_cell_matches_level_kernel(name, local, sr, band):
+    cm, g, l = models(name)
+    a, b = scan.Scanner(l if local else g), scan.Scanner(l if local else g)
+    b.set_kernel(KERNEL_LEVEL)
+    for n, chunk in ((40, 0), (700, 0), (1500, 130)):
+        dsq = frame(seq_of(cm, n, n))
+        a.set_shape(0, 0, chunk, 0)
+        ca, cb = a.scan_cells(sr, band, dsq, 1, n, -30.0), b.scan_cells(sr, band, dsq, 1, n, -30.0)
+        assert (a.stats()["kernel"], b.stats()["kernel"]) == (DIAG, KERNEL_LEVEL)
+        assert ca == cb
+
+
+@pytest.mark.parametrize("sr", [CYK_F32, INSIDE_I32])
+@pytest.mark.parametrize("null3", [False, True])
+def test_calibration_scan_matches_level_kernel(sr, null3):
+    cm, g, l = models("trna")
+    buf = frame(seq_of(cm, 1500, 9))
+    w = np.array([(0, 1, 1500), (0, 500, 1200), (0, 1, 40), (0, 900, 899)], N.WINDOW_DTYPE)
+    for c in (g, l):
+        a, b = scan.Scanner(c), scan.Scanner(c)
+        b.set_kernel(KERNEL_LEVEL)
+        x = a.calibrate_scan_batch(sr, QDB2, buf, w, null3)
+        y = b.calibrate_scan_batch(sr, QDB2, buf, w, null3)
+        assert len(x) > 0 and x.tobytes() == y.tobytes()
