@@ -628,7 +628,7 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
             set_error("diagonal kernel cannot be resident");
             return CMGPU_EDEVICE;
         }
-        best_c = occ;
+        best_c = ws->ctas_per_sm > 0 ? std::min(ws->ctas_per_sm, occ) : occ;
         ws->stats.lanes = best_l;
     }
 

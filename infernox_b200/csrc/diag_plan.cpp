@@ -8,20 +8,6 @@
 
 namespace cmx {
 
-namespace {
-
-// A score a floating maximum treats as the reference's `a >= b ? a : b` does
-// in every sum and comparison: not NaN, not +inf, not -0 (with none of these
-// in the tables no sum yields one).
-bool plain_float(uint32_t bits) {
-    float f;
-    std::memcpy(&f, &bits, 4);
-    if (std::isnan(f) || (std::isinf(f) && f > 0)) return false;
-    return !(f == 0.0f && std::signbit(f));
-}
-
-}  // namespace
-
 bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp, std::string *why) {
     auto fail = [&](const char *m) {
         if (why) *why = m;
@@ -31,60 +17,19 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
     dp = DiagPlan();
     if (p.semiring != CMGPU_INSIDE_I32) {
         for (const auto *t : {&p.tsc, &p.endsc, &p.beginsc_all, &p.esc, &p.el_sca})
-            for (uint32_t x : *t)
-                if (!plain_float(x)) return fail("score tables hold -0, NaN or +inf");
+            for (uint32_t x : *t) {
+                float f;
+                std::memcpy(&f, &x, 4);
+                if (!plain_float(f)) return fail("score tables hold -0, NaN or +inf");
+            }
     }
-    // nodes from the unique state ids
-    std::vector<NodeShape> shape;
-    std::vector<int> v0s, node_of(M, -1);
-    for (int v = 0; v < M;) {
-        NodeShape ns;
-        if (!node_shape(cm->stid[v], ns)) return fail("state list does not start a node where expected");
-        if (v + ns.nst > M) return fail("truncated node");
-        static const int TYPES[20] = {S_ST, IL_ST, IR_ST, S_ST, S_ST, IL_ST, MP_ST, ML_ST, MR_ST, D_ST,
-                                      IL_ST, IR_ST, ML_ST, D_ST, IL_ST, MR_ST, D_ST, IR_ST, B_ST, E_ST};
-        for (int q = 0; q < ns.nst; q++) {
-            if (cm->stid[v + q] != ns.ids[q] || cm->sttype[v + q] != TYPES[ns.ids[q]])
-                return fail("unexpected state inside a node");
-            node_of[v + q] = (int)shape.size();
-        }
-        shape.push_back(ns);
-        v0s.push_back(v);
-        v += ns.nst;
-    }
+    std::vector<NodeTopo> shape;
+    const char *msg = nullptr;
+    if (!node_topology(cm, shape, &msg)) return fail(msg);
     const int nn = (int)shape.size();
-    if (shape[0].type != ROOT_ND || shape[nn - 1].type != END_ND) return fail("first node is not ROOT or last not END");
-    auto is_insert = [&](int v) { return cm->sttype[v] == IL_ST || cm->sttype[v] == IR_ST; };
-    std::vector<int> bif_l(nn, -1), bif_r(nn, -1);  // BIF node -> BEGL / BEGR node
-    std::vector<char> claimed(nn, 0);               // BEGL / BEGR nodes with their bifurcation
-    for (int v = 0; v < M; v++) {
-        const int st = cm->sttype[v], n = node_of[v];
-        if (st == E_ST) continue;
-        if (st == B_ST) {
-            const int wl = cm->cfirst[v], y = cm->cnum[v];
-            if (wl != v + 1 || cm->stid[wl] != UID_BEGL_S || y <= wl || y >= M || cm->stid[y] != UID_BEGR_S)
-                return fail("bifurcation children are not BEGL_S / BEGR_S");
-            bif_l[n] = node_of[wl];
-            bif_r[n] = node_of[y];
-            if (claimed[bif_l[n]] || claimed[bif_r[n]]) return fail("a subtree belongs to two bifurcations");
-            claimed[bif_l[n]] = claimed[bif_r[n]] = 1;
-            continue;
-        }
-        if (n + 1 >= nn) return fail("a non-END last node");
-        if (shape[n + 1].type == BEGL_ND || shape[n + 1].type == BEGR_ND || shape[n + 1].type == ROOT_ND)
-            return fail("a node is followed by a subtree start");
-        const int v0 = v0s[n];
-        int k = 0;
-        bool ok = true;
-        auto kid = [&](int u) { ok = ok && k < cm->cnum[v] && cm->cfirst[v] + k == u, k++; };
-        for (int q = 0; q < shape[n].nst; q++)
-            if (is_insert(v0 + q) && !(is_insert(v) && v0 + q < v)) kid(v0 + q);
-        for (int q = 0; q < shape[n + 1].nsplit; q++) kid(v0s[n + 1] + q);
-        if (!ok || k != cm->cnum[v]) return fail("children are not the node's inserts and the next node's split states");
-    }
+    std::vector<int> node_of(M, 0);
     for (int n = 0; n < nn; n++)
-        if ((shape[n].type == BEGL_ND || shape[n].type == BEGR_ND) && !claimed[n])
-            return fail("a subtree start without its bifurcation");
+        for (int q = 0; q < shape[n].nst; q++) node_of[shape[n].v0 + q] = n;
     // spans a node stores: its states' bands and every span a parent or a
     // bifurcation reads
     Bands b = select_bands(cm, qdbidx);
@@ -100,8 +45,8 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
         cover(n, b.dn[v], b.dxcap[v]);
         if (st == B_ST) {
             const int wl = cm->cfirst[v], y = cm->cnum[v];
-            cover(bif_l[n], std::max(0, std::min(b.dmin[wl], W)), std::min(b.dmax[wl], W));
-            cover(bif_r[n], std::max(0, std::min(b.dmin[y], W)), std::min(b.dmax[y], W));
+            cover(shape[n].begl, std::max(0, std::min(b.dmin[wl], W)), std::min(b.dmax[wl], W));
+            cover(shape[n].begr, std::max(0, std::min(b.dmin[y], W)), std::min(b.dmax[y], W));
         } else {
             const int sd = v == 0 ? 0 : state_delta(st);
             cover(n + 1, b.dn[v] - sd, b.dxcap[v] - sd);
@@ -137,13 +82,11 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
         if (shape[n].type == END_ND) continue;
         buf[n] = t++ % 3;
         DgNode d{};
-        d.v0 = v0s[n];
+        d.v0 = shape[n].v0;
         d.type = (int16_t)shape[n].type;
         d.nn = n + 1 < nn ? (int16_t)shape[n + 1].nsplit : 1;
         d.next_end = n + 1 < nn && shape[n + 1].type == END_ND;
-        const int pt = n > 0 ? shape[n - 1].type : BIF_ND;
-        const bool child_of_prev = n > 0 && shape[n].type != BEGL_ND && shape[n].type != BEGR_ND;
-        d.need_left = child_of_prev && (pt == MATP_ND || pt == MATR_ND || pt == ROOT_ND);
+        d.need_left = shape[n].need_left;
         d.rlo = lo[n];
         d.rhi = hi[n];
         if (n + 1 < nn) d.clo = lo[n + 1], d.chi = hi[n + 1];
@@ -153,7 +96,7 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
         d.bnd_off = off;
         off += (int64_t)(hi[n] - lo[n] + 1) * (DG_SLOTS + 2);
         for (int q = 0; q < shape[n].nst; q++) {
-            const int v = v0s[n] + q;
+            const int v = shape[n].v0 + q;
             const StateDev &s = p.states[v];
             const bool live = s.dxcap >= s.dn;
             d.dn[q] = live ? s.dn : (int16_t)32767;
@@ -162,13 +105,13 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
             if (s.flags & SF_ENDSC) d.endmask |= 1 << q;
             if (live && (s.flags & SF_BEGIN)) d.beginmask |= 1 << q;
         }
-        if (d.next_end) d.cinit0 = p.init0[v0s[n + 1]];
+        if (d.next_end) d.cinit0 = p.init0[shape[n + 1].v0];
         if (shape[n].type == BIF_ND) {
-            const int wl = cm->cfirst[v0s[n]], y = cm->cnum[v0s[n]];
-            d.begl_lo = lo[bif_l[n]];
-            d.begr_lo = lo[bif_r[n]];
-            d.begl_off = deck[bif_l[n]];
-            d.begr_off = deck[bif_r[n]];
+            const int wl = cm->cfirst[d.v0], y = cm->cnum[d.v0];
+            d.begl_lo = lo[shape[n].begl];
+            d.begr_lo = lo[shape[n].begr];
+            d.begl_off = deck[shape[n].begl];
+            d.begr_off = deck[shape[n].begr];
             d.kdn_y = std::min(b.dmin[y], W);
             d.kdx_y = std::min(b.dmax[y], W);
             d.kdn_w = std::min(b.dmin[wl], W);

@@ -2,6 +2,7 @@
 // diag_plan.cpp).
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
@@ -69,6 +70,94 @@ inline bool node_shape(int first_id, NodeShape &ns) {
     case UID_END_E: ns = {END_ND, 1, 1, {UID_END_E}}; return true;
     default: return false;
     }
+}
+
+// One node of a CM with cm_from_guide's topology.
+struct NodeTopo {
+    int v0, type, nst, nsplit;
+    int begl = -1, begr = -1;  // BIF: the nodes of its two subtrees
+    bool need_left = false;    // the parent node reads column j-1 of the split states
+};
+
+// The nodes of `cm` in order, if a state's children are its node's own
+// inserts followed by the next node's split states, and a bifurcation's are
+// BEGL_S and BEGR_S; else false with the reason in `why`.
+inline bool node_topology(const cmgpu_cm *cm, std::vector<NodeTopo> &out, const char **why) {
+    auto fail = [&](const char *m) {
+        if (why) *why = m;
+        return false;
+    };
+    const int M = cm->M;
+    std::vector<NodeShape> shape;
+    std::vector<int> node_of(M, -1);
+    out.clear();
+    for (int v = 0; v < M;) {
+        NodeShape ns;
+        if (!node_shape(cm->stid[v], ns)) return fail("state list does not start a node where expected");
+        if (v + ns.nst > M) return fail("truncated node");
+        static const int TYPES[20] = {S_ST, IL_ST, IR_ST, S_ST, S_ST, IL_ST, MP_ST, ML_ST, MR_ST, D_ST,
+                                      IL_ST, IR_ST, ML_ST, D_ST, IL_ST, MR_ST, D_ST, IR_ST, B_ST, E_ST};
+        for (int q = 0; q < ns.nst; q++) {
+            if (cm->stid[v + q] != ns.ids[q] || cm->sttype[v + q] != TYPES[ns.ids[q]])
+                return fail("unexpected state inside a node");
+            node_of[v + q] = (int)shape.size();
+        }
+        shape.push_back(ns);
+        NodeTopo t;
+        t.v0 = v;
+        t.type = ns.type;
+        t.nst = ns.nst;
+        t.nsplit = ns.nsplit;
+        out.push_back(t);
+        v += ns.nst;
+    }
+    const int nn = (int)shape.size();
+    if (nn < 2 || shape[0].type != ROOT_ND || shape[nn - 1].type != END_ND)
+        return fail("first node is not ROOT or last not END");
+    auto is_insert = [&](int v) { return cm->sttype[v] == IL_ST || cm->sttype[v] == IR_ST; };
+    std::vector<char> claimed(nn, 0);  // BEGL / BEGR nodes with their bifurcation
+    for (int v = 0; v < M; v++) {
+        const int st = cm->sttype[v], n = node_of[v];
+        if (st == E_ST) continue;
+        if (st == B_ST) {
+            const int wl = cm->cfirst[v], y = cm->cnum[v];
+            if (wl != v + 1 || cm->stid[wl] != UID_BEGL_S || y <= wl || y >= M || cm->stid[y] != UID_BEGR_S)
+                return fail("bifurcation children are not BEGL_S / BEGR_S");
+            out[n].begl = node_of[wl];
+            out[n].begr = node_of[y];
+            if (claimed[out[n].begl] || claimed[out[n].begr]) return fail("a subtree belongs to two bifurcations");
+            claimed[out[n].begl] = claimed[out[n].begr] = 1;
+            continue;
+        }
+        if (n + 1 >= nn) return fail("a non-END last node");
+        if (shape[n + 1].type == BEGL_ND || shape[n + 1].type == BEGR_ND || shape[n + 1].type == ROOT_ND)
+            return fail("a node is followed by a subtree start");
+        const int v0 = out[n].v0;
+        int k = 0;
+        bool ok = true;
+        auto kid = [&](int u) { ok = ok && k < cm->cnum[v] && cm->cfirst[v] + k == u, k++; };
+        for (int q = 0; q < shape[n].nst; q++)
+            if (is_insert(v0 + q) && !(is_insert(v) && v0 + q < v)) kid(v0 + q);
+        for (int q = 0; q < shape[n + 1].nsplit; q++) kid(out[n + 1].v0 + q);
+        if (!ok || k != cm->cnum[v])
+            return fail("children are not the node's inserts and the next node's split states");
+        if (cm->sttype[v] != S_ST || n == 0) {
+            const int pt = shape[n].type;
+            if (pt == MATP_ND || pt == MATR_ND || pt == ROOT_ND) out[n + 1].need_left = true;
+        }
+    }
+    for (int n = 0; n < nn; n++)
+        if ((shape[n].type == BEGL_ND || shape[n].type == BEGR_ND) && !claimed[n])
+            return fail("a subtree start without its bifurcation");
+    return true;
+}
+
+// A score a floating maximum treats as the reference's `a >= b ? a : b` does
+// in every sum and comparison: not NaN, not +inf, not -0 (with none of these
+// in the tables no sum yields one).
+inline bool plain_float(float f) {
+    if (std::isnan(f) || (std::isinf(f) && f > 0)) return false;
+    return !(f == 0.0f && std::signbit(f));
 }
 
 }  // namespace cmx

@@ -60,6 +60,8 @@
 
 #include "devbuf.h"
 #include "model_internal.h"
+#include "plan_util.h"
+#include "trq_diag.h"
 #include "trunc_report.h"
 
 namespace cmx {
@@ -69,6 +71,9 @@ struct TrqDev {
     int8_t *sttype = nullptr, *kind = nullptr;
     int32_t *cfirst = nullptr, *cnum = nullptr, *begl_idx = nullptr;
     uint32_t *tsc[2] = {nullptr, nullptr}, *esc[2] = {nullptr, nullptr}, *init_sc[2] = {nullptr, nullptr};
+    uint32_t *endsc[2] = {nullptr, nullptr}, *el[2] = {nullptr, nullptr};  // the diagonal kernel's init_sc: el[d] + endsc[v]
+    bool esc_plain = true;   // f32 emission scores: no NaN, +inf or -0
+    int64_t esc_best = 0;    // largest integer emission score
     std::vector<int> level, kind_h, begl_h;
     int nlev = 0, nbegl = 0;
     DevArena arena;
@@ -92,6 +97,8 @@ void trq_free(TrqDev *t) {
         cudaFree(t->tsc[s]);
         cudaFree(t->esc[s]);
         cudaFree(t->init_sc[s]);
+        cudaFree(t->endsc[s]);
+        cudaFree(t->el[s]);
     }
     delete t;
 }
@@ -107,17 +114,8 @@ constexpr int END_E = 19;  // unique state id of END states (src/constants.rs)
 // what a state does in the column loop
 enum { K_SKIP = 0, K_B, K_BEGL, K_IL, K_ML, K_MRIR, K_MP, K_SD };
 
-struct Win {
-    int64_t dsq_off;
-    int32_t i0, j0, w, idx;  // idx: the window's index in the caller's batch
-};
-
-struct Res {
-    float vsc;
-    int32_t vmode;
-    float bsc_full;
-    int32_t pad;
-};
+using trqd::Res;
+using trqd::Win;
 
 struct Tab {
     const int8_t *sttype, *kind;
@@ -741,10 +739,14 @@ int trq_semiring_tables(cmgpu_model *m, TrqDev *q, bool ins) {
     std::vector<uint32_t> tsc((size_t)M * MAXC), esc((size_t)M * ESC), init((size_t)M * (W + 1));
     for (size_t x = 0; x < tsc.size(); x++) tsc[x] = ins ? iw(c.itsc[x]) : fw(c.tsc[x]);
     for (size_t x = 0; x < esc.size(); x++) esc[x] = ins ? iw(c.ioesc[x]) : fw(c.oesc[x]);
+    std::vector<uint32_t> elw(W + 1), endw(M);
+    for (int v = 0; v < M; v++) endw[v] = ins ? iw(c.iendsc[v]) : fw(c.endsc[v]);
     if (ins) {
         std::vector<int32_t> el(W + 1);
         el[0] = 0;
         for (int d = 1; d <= W; d++) el[d] = (int32_t)((uint32_t)el[d - 1] + (uint32_t)c.view.iel_selfsc);
+        for (int d = 0; d <= W; d++) elw[d] = iw(el[d]);
+        for (size_t x = 0; x < esc.size(); x++) q->esc_best = std::max<int64_t>(q->esc_best, c.ioesc[x]);
         for (int v = 0; v < M; v++)
             for (int d = 0; d <= W; d++)
                 init[(size_t)v * (W + 1) + d] =
@@ -753,6 +755,8 @@ int trq_semiring_tables(cmgpu_model *m, TrqDev *q, bool ins) {
         std::vector<float> el(W + 1);
         el[0] = 0.0f;
         for (int d = 1; d <= W; d++) el[d] = el[d - 1] + c.view.el_selfsc;
+        for (int d = 0; d <= W; d++) elw[d] = fw(el[d]);
+        for (size_t x = 0; x < esc.size(); x++) q->esc_plain = q->esc_plain && plain_float(c.oesc[x]);
         for (int v = 0; v < M; v++)
             for (int d = 0; d <= W; d++)
                 init[(size_t)v * (W + 1) + d] =
@@ -760,6 +764,8 @@ int trq_semiring_tables(cmgpu_model *m, TrqDev *q, bool ins) {
     }
     int rc = upload_arr(&q->tsc[s], tsc.data(), tsc.size());
     if (!rc) rc = upload_arr(&q->esc[s], esc.data(), esc.size());
+    if (!rc) rc = upload_arr(&q->endsc[s], endw.data(), endw.size());
+    if (!rc) rc = upload_arr(&q->el[s], elw.data(), elw.size());
     if (!rc) rc = upload_arr(&q->init_sc[s], init.data(), init.size());
     if (rc) set_error("truncated QDB scan: uploading the score tables failed");
     return rc;
@@ -844,50 +850,6 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
         const int dmax = qdbidx == 0 ? W : (qdbidx == 1 ? c.dmax1[v] : c.dmax2[v]);
         dxcap[v] = std::min(dmax, W);
     }
-    // the wavefront: unit (level l, chunk c) in step l + c over the levels
-    // that hold work, the ROOT cells as one more level; a step's units sorted
-    // by chunk (a column with fewer rows takes a prefix: cu_off / il_off),
-    // then B units first and the rest by kind
-    std::vector<int> lmap(std::max(q->nlev, 1), -1);
-    for (int v = 1; v < M; v++)
-        if (q->kind_h[v] != trq::K_SKIP && dxcap[v] >= 1) lmap[q->level[v]] = 0;
-    int nl = 0;
-    for (int &x : lmap)
-        if (x == 0) x = nl++;
-    const int NC = (W + trq::CH - 1) / trq::CH;
-    const int nstep = nl + NC;
-    struct U {
-        int c, key, v, d0;
-    };
-    std::vector<std::vector<U>> sc_cells(nstep), sc_il(nstep);
-    for (int v = 1; v < M; v++) {
-        const int k = q->kind_h[v];
-        if (k == trq::K_SKIP || dxcap[v] < 1) continue;
-        for (int d0 = 1, ch = 0; d0 <= dxcap[v]; d0 += trq::CH, ch++) {
-            const int sp = lmap[q->level[v]] + ch;
-            (k == trq::K_IL ? sc_il : sc_cells)[sp].push_back(U{ch, k == trq::K_B ? 0 : k + 1, v, d0});
-        }
-    }
-    std::vector<int2> units, il_units;
-    std::vector<int32_t> cu_off((size_t)nstep * (NC + 1)), il_off((size_t)nstep * (NC + 1));
-    auto lay = [&](std::vector<U> &L, std::vector<int2> &out, int32_t *off) {
-        std::sort(L.begin(), L.end(), [](const U &a, const U &b) {
-            if (a.c != b.c) return a.c < b.c;
-            if (a.key != b.key) return a.key < b.key;
-            if (a.v != b.v) return a.v < b.v;
-            return a.d0 < b.d0;
-        });
-        size_t x = 0;
-        for (int c = 0; c <= NC; c++) {
-            while (x < L.size() && L[x].c < c) x++;
-            off[c] = (int32_t)(out.size() + x);
-        }
-        for (const U &u : L) out.push_back(int2{u.v, u.d0});
-    };
-    for (int sp = 0; sp < nstep; sp++) {
-        lay(sc_cells[sp], units, cu_off.data() + (size_t)sp * (NC + 1));
-        lay(sc_il[sp], il_units, il_off.data() + (size_t)sp * (NC + 1));
-    }
     std::vector<int32_t> pbeg;
     std::vector<uint32_t> lm((size_t)M * KP), rm((size_t)M * KP), pty(M), base;
     for (int y = 1; y < M; y++)
@@ -940,75 +902,197 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     if (wl.empty()) return CMGPU_OK;
 
     const int nw = (int)wl.size();
-    for (const trq::Win &x : wl)
-        if ((int64_t)(x.j0 - x.i0 + 1) * nstep >= INT_MAX) {
-            set_error("truncated QDB scan: window too long for the column progress counters");
-            return CMGPU_EINVAL;
-        }
-    const int W1 = wmax + 1;
-    const int nbk = std::max(q->nbegl, 1);  // the kernel's BEGL deck count (one unused deck without BEGL states)
-    const int64_t nplane = trq::NW + 1;
-    const int64_t deck_stride =
-        ((int64_t)4 * nplane * M * W1 + (int64_t)8 * W1 + (int64_t)3 * (W1 + trq::NW) * nbk * W1 + 63) / 64 * 64;
-    const size_t smem = (size_t)(W + 1) * 12 + (ins ? ((size_t)m->ilog_nz * 2 + 16) : 0);
-    auto kfn = ins ? trq::trq_kernel<true> : trq::trq_kernel<false>;
-    TRQ_TRY(cmx::allow_max_dynamic_smem(kfn));
-    int occ = 0, nsm = 0;
-    TRQ_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, trq::THREADS, smem));
-    TRQ_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
-    if (occ < 1) {
-        set_error("truncated QDB scan: the kernel does not fit on an SM (W too large)");
-        return CMGPU_EINVAL;
-    }
-    const int64_t budget = q->deck_budget;  // bytes of decks
-    int64_t grid = std::min<int64_t>({(int64_t)nw, (int64_t)occ * nsm, std::max<int64_t>(1, budget / (deck_stride * 4))});
-
+    const bool fill_l = pass_idx == 3 || pass_idx == 4 || pass_idx == 5;
+    const bool fill_r = pass_idx == 2 || pass_idx == 4 || pass_idx == 5;
+    const bool fill_t = pass_idx == 4 || pass_idx == 5;
     DevArena &ar = q->arena;
-    int2 *d_units, *d_il;
-    int32_t *d_cuoff, *d_iloff, *d_dx, *d_pbeg;
-    uint32_t *d_lm, *d_rm, *d_pty, *d_base, *d_decks;
+    uint32_t *d_lm, *d_rm, *d_pty, *d_decks;
     trq::Win *d_win;
     uint8_t *d_dsq;
     trq::Res *d_res;
     int *d_queue;
     unsigned long long *d_nc;
-    if (ar.get(0, &d_units, sizeof(int2) * std::max<size_t>(units.size(), 1)) ||
-        ar.get(1, &d_cuoff, sizeof(int32_t) * cu_off.size()) || ar.get(2, &d_dx, sizeof(int32_t) * M) ||
-        ar.get(15, &d_il, sizeof(int2) * std::max<size_t>(il_units.size(), 1)) ||
-        ar.get(16, &d_iloff, sizeof(int32_t) * il_off.size()) ||
-        ar.get(3, &d_pbeg, sizeof(int32_t) * (pbeg.size() + 1)) || ar.get(4, &d_lm, sizeof(uint32_t) * lm.size()) ||
-        ar.get(5, &d_rm, sizeof(uint32_t) * rm.size()) || ar.get(6, &d_pty, sizeof(uint32_t) * M) ||
-        ar.get(7, &d_base, sizeof(uint32_t) * base.size()) || ar.get(8, &d_win, sizeof(trq::Win) * nw) ||
+    if (ar.get(4, &d_lm, sizeof(uint32_t) * lm.size()) || ar.get(5, &d_rm, sizeof(uint32_t) * rm.size()) ||
+        ar.get(6, &d_pty, sizeof(uint32_t) * M) || ar.get(8, &d_win, sizeof(trq::Win) * nw) ||
         ar.get(9, &d_dsq, (size_t)dsq_len) || ar.get(10, &d_res, sizeof(trq::Res) * nwin) ||
-        ar.get(11, &d_decks, sizeof(uint32_t) * (size_t)deck_stride * (size_t)grid) ||
         ar.get(12, &d_queue, sizeof(int) * 2) || ar.get(13, &d_nc, sizeof(unsigned long long))) {
         set_error("truncated QDB scan: device allocation failed");
         return CMGPU_ENOMEM;
     }
-    if (!units.empty())
-        TRQ_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int2) * units.size(), cudaMemcpyHostToDevice, st));
-    if (!il_units.empty())
-        TRQ_TRY(cudaMemcpyAsync(d_il, il_units.data(), sizeof(int2) * il_units.size(), cudaMemcpyHostToDevice, st));
-    TRQ_TRY(cudaMemcpyAsync(d_cuoff, cu_off.data(), sizeof(int32_t) * cu_off.size(), cudaMemcpyHostToDevice, st));
-    TRQ_TRY(cudaMemcpyAsync(d_iloff, il_off.data(), sizeof(int32_t) * il_off.size(), cudaMemcpyHostToDevice, st));
-    TRQ_TRY(cudaMemcpyAsync(d_dx, dxcap.data(), sizeof(int32_t) * M, cudaMemcpyHostToDevice, st));
-    if (!pbeg.empty())
-        TRQ_TRY(cudaMemcpyAsync(d_pbeg, pbeg.data(), sizeof(int32_t) * pbeg.size(), cudaMemcpyHostToDevice, st));
     TRQ_TRY(cudaMemcpyAsync(d_lm, lm.data(), sizeof(uint32_t) * lm.size(), cudaMemcpyHostToDevice, st));
     TRQ_TRY(cudaMemcpyAsync(d_rm, rm.data(), sizeof(uint32_t) * rm.size(), cudaMemcpyHostToDevice, st));
     TRQ_TRY(cudaMemcpyAsync(d_pty, pty.data(), sizeof(uint32_t) * M, cudaMemcpyHostToDevice, st));
-    TRQ_TRY(cudaMemcpyAsync(d_base, base.data(), sizeof(uint32_t) * base.size(), cudaMemcpyHostToDevice, st));
     TRQ_TRY(cudaMemcpyAsync(d_win, wl.data(), sizeof(trq::Win) * nw, cudaMemcpyHostToDevice, st));
     TRQ_TRY(cudaMemcpyAsync(d_dsq, dsq_all, (size_t)dsq_len, cudaMemcpyHostToDevice, st));
-    const bool fill_l = pass_idx == 3 || pass_idx == 4 || pass_idx == 5;
-    const bool fill_r = pass_idx == 2 || pass_idx == 4 || pass_idx == 5;
-    const bool fill_t = pass_idx == 4 || pass_idx == 5;
-    const trq::Tab tab{q->sttype, q->kind, q->cfirst, q->cnum, d_dx, q->begl_idx, d_pbeg, d_cuoff, d_iloff,
-                       d_units, d_il, q->tsc[s], q->esc[s], d_lm, d_rm, d_pty, q->init_sc[s], d_base, m->ilog,
-                       m->ilog_nz, M, W, nbk, (int)pbeg.size(), qdbidx == 0, fill_l, fill_r, fill_t,
-                       nl, NC, nstep, q->stall_col};
+    int nsm = 0;
+    TRQ_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
+    const int64_t budget = q->deck_budget;  // bytes of decks
+
+    // The diagonal kernel takes every model with cm_from_guide's node layout;
+    // the column wavefront takes the others, and the calls of the test hook,
+    // which stalls one of its columns.
+    std::vector<trqd::Node> nodes;
+    trqd::Params dgp{};
+    std::vector<char> skip(M, 0);
+    for (int v = 1; v < M; v++) skip[v] = q->kind_h[v] == trq::K_SKIP;
+    const bool diag = q->stall_col < 0 &&
+                      trqd::build(&c.view, ins, dxcap, skip, pty, pbeg, lm, rm, base, q->begl_h, q->esc_plain,
+                                  q->esc_best, nodes, &dgp.nbif);
+    std::vector<int2> units, il_units;
+    std::vector<int32_t> cu_off, il_off;
+    trq::Tab tab{};
+    int64_t grid = 0, deck_stride = 0;
+    size_t smem = 0;
+    int warps = 0;
+    auto kfn = ins ? trq::trq_kernel<true> : trq::trq_kernel<false>;
+    if (diag) {
+        dgp.nnodes = (int)nodes.size();
+        dgp.tsc = q->tsc[s];
+        dgp.esc = q->esc[s];
+        dgp.lm = d_lm;
+        dgp.rm = d_rm;
+        dgp.pty = d_pty;
+        dgp.endsc = q->endsc[s];
+        dgp.el = q->el[s];
+        dgp.W = W;
+        dgp.W1 = wmax + 1;
+        dgp.dx0 = std::min(dxcap[0], wmax);
+        dgp.inside = ins;
+        dgp.fill_l = fill_l;
+        dgp.fill_r = fill_r;
+        dgp.fill_t = fill_t;
+        dgp.nonbanded = qdbidx == 0;
+        dgp.ilog = m->ilog;
+        dgp.ilog_nz = m->ilog_nz;
+        dgp.dsq = d_dsq;
+        dgp.wins = d_win;
+        dgp.nwin = nw;
+        dgp.queue = d_queue;
+        dgp.cutoff = cutoff;
+        dgp.ncand = d_nc;
+        dgp.res = d_res;
+        // no more warps than the longest window has columns
+        const int longest = wl[0].j0 - wl[0].i0 + 1;
+        warps = std::min(trqd::MAX_WARPS, (longest + 31) / 32);
+        dgp.ring_cols = (dgp.W1 + trqd::COLS + 31) & ~31;
+        dgp.ring_len = 1;
+        while (dgp.ring_len < dgp.W1 + 64 * warps) dgp.ring_len <<= 1;
+        dgp.region_words = trqd::region_words(dgp);
+        const int occ = trqd::occupancy(dgp, warps);
+        if (occ < 1) {
+            set_error("truncated QDB scan: the kernel does not fit on an SM (W too large)");
+            return CMGPU_EINVAL;
+        }
+        grid = std::min<int64_t>(
+            {(int64_t)nw, (int64_t)occ * nsm, std::max<int64_t>(1, budget / (dgp.region_words * 4))});
+        trqd::Node *d_nodes;
+        if (ar.get(11, &d_decks, sizeof(uint32_t) * (size_t)dgp.region_words * (size_t)grid) ||
+            ar.get(0, &d_nodes, sizeof(trqd::Node) * nodes.size())) {
+            set_error("truncated QDB scan: device allocation failed");
+            return CMGPU_ENOMEM;
+        }
+        TRQ_TRY(cudaMemcpyAsync(d_nodes, nodes.data(), sizeof(trqd::Node) * nodes.size(), cudaMemcpyHostToDevice, st));
+        dgp.nodes = d_nodes;
+        dgp.region = d_decks;
+    } else {
+        // the wavefront: unit (level l, chunk c) in step l + c over the levels
+        // that hold work, the ROOT cells as one more level; a step's units sorted
+        // by chunk (a column with fewer rows takes a prefix: cu_off / il_off),
+        // then B units first and the rest by kind
+        std::vector<int> lmap(std::max(q->nlev, 1), -1);
+        for (int v = 1; v < M; v++)
+            if (q->kind_h[v] != trq::K_SKIP && dxcap[v] >= 1) lmap[q->level[v]] = 0;
+        int nl = 0;
+        for (int &x : lmap)
+            if (x == 0) x = nl++;
+        const int NC = (W + trq::CH - 1) / trq::CH;
+        const int nstep = nl + NC;
+        struct U {
+            int c, key, v, d0;
+        };
+        std::vector<std::vector<U>> sc_cells(nstep), sc_il(nstep);
+        for (int v = 1; v < M; v++) {
+            const int k = q->kind_h[v];
+            if (k == trq::K_SKIP || dxcap[v] < 1) continue;
+            for (int d0 = 1, ch = 0; d0 <= dxcap[v]; d0 += trq::CH, ch++) {
+                const int sp = lmap[q->level[v]] + ch;
+                (k == trq::K_IL ? sc_il : sc_cells)[sp].push_back(U{ch, k == trq::K_B ? 0 : k + 1, v, d0});
+            }
+        }
+        cu_off.resize((size_t)nstep * (NC + 1));
+        il_off.resize((size_t)nstep * (NC + 1));
+        auto lay = [&](std::vector<U> &L, std::vector<int2> &out, int32_t *off) {
+            std::sort(L.begin(), L.end(), [](const U &a, const U &b) {
+                if (a.c != b.c) return a.c < b.c;
+                if (a.key != b.key) return a.key < b.key;
+                if (a.v != b.v) return a.v < b.v;
+                return a.d0 < b.d0;
+            });
+            size_t x = 0;
+            for (int c = 0; c <= NC; c++) {
+                while (x < L.size() && L[x].c < c) x++;
+                off[c] = (int32_t)(out.size() + x);
+            }
+            for (const U &u : L) out.push_back(int2{u.v, u.d0});
+        };
+        for (int sp = 0; sp < nstep; sp++) {
+            lay(sc_cells[sp], units, cu_off.data() + (size_t)sp * (NC + 1));
+            lay(sc_il[sp], il_units, il_off.data() + (size_t)sp * (NC + 1));
+        }
+        for (const trq::Win &x : wl)
+            if ((int64_t)(x.j0 - x.i0 + 1) * nstep >= INT_MAX) {
+                set_error("truncated QDB scan: window too long for the column progress counters");
+                return CMGPU_EINVAL;
+            }
+        const int W1 = wmax + 1;
+        const int nbk = std::max(q->nbegl, 1);  // the kernel's BEGL deck count (one unused deck without BEGL states)
+        const int64_t nplane = trq::NW + 1;
+        deck_stride =
+            ((int64_t)4 * nplane * M * W1 + (int64_t)8 * W1 + (int64_t)3 * (W1 + trq::NW) * nbk * W1 + 63) / 64 * 64;
+        smem = (size_t)(W + 1) * 12 + (ins ? ((size_t)m->ilog_nz * 2 + 16) : 0);
+        TRQ_TRY(cmx::allow_max_dynamic_smem(kfn));
+        int occ = 0;
+        TRQ_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, trq::THREADS, smem));
+        if (occ < 1) {
+            set_error("truncated QDB scan: the kernel does not fit on an SM (W too large)");
+            return CMGPU_EINVAL;
+        }
+        grid = std::min<int64_t>({(int64_t)nw, (int64_t)occ * nsm, std::max<int64_t>(1, budget / (deck_stride * 4))});
+
+        int2 *d_units, *d_il;
+        int32_t *d_cuoff, *d_iloff, *d_dx, *d_pbeg;
+        uint32_t *d_base;
+        if (ar.get(0, &d_units, sizeof(int2) * std::max<size_t>(units.size(), 1)) ||
+            ar.get(1, &d_cuoff, sizeof(int32_t) * cu_off.size()) || ar.get(2, &d_dx, sizeof(int32_t) * M) ||
+            ar.get(15, &d_il, sizeof(int2) * std::max<size_t>(il_units.size(), 1)) ||
+            ar.get(16, &d_iloff, sizeof(int32_t) * il_off.size()) ||
+            ar.get(3, &d_pbeg, sizeof(int32_t) * (pbeg.size() + 1)) ||
+            ar.get(7, &d_base, sizeof(uint32_t) * base.size()) ||
+            ar.get(11, &d_decks, sizeof(uint32_t) * (size_t)deck_stride * (size_t)grid)) {
+            set_error("truncated QDB scan: device allocation failed");
+            return CMGPU_ENOMEM;
+        }
+        if (!units.empty())
+            TRQ_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int2) * units.size(), cudaMemcpyHostToDevice, st));
+        if (!il_units.empty())
+            TRQ_TRY(cudaMemcpyAsync(d_il, il_units.data(), sizeof(int2) * il_units.size(), cudaMemcpyHostToDevice, st));
+        TRQ_TRY(cudaMemcpyAsync(d_cuoff, cu_off.data(), sizeof(int32_t) * cu_off.size(), cudaMemcpyHostToDevice, st));
+        TRQ_TRY(cudaMemcpyAsync(d_iloff, il_off.data(), sizeof(int32_t) * il_off.size(), cudaMemcpyHostToDevice, st));
+        TRQ_TRY(cudaMemcpyAsync(d_dx, dxcap.data(), sizeof(int32_t) * M, cudaMemcpyHostToDevice, st));
+        if (!pbeg.empty())
+            TRQ_TRY(cudaMemcpyAsync(d_pbeg, pbeg.data(), sizeof(int32_t) * pbeg.size(), cudaMemcpyHostToDevice, st));
+        TRQ_TRY(cudaMemcpyAsync(d_base, base.data(), sizeof(uint32_t) * base.size(), cudaMemcpyHostToDevice, st));
+        tab = trq::Tab{q->sttype, q->kind, q->cfirst, q->cnum, d_dx, q->begl_idx, d_pbeg, d_cuoff, d_iloff,
+                           d_units, d_il, q->tsc[s], q->esc[s], d_lm, d_rm, d_pty, q->init_sc[s], d_base, m->ilog,
+                           m->ilog_nz, M, W, nbk, (int)pbeg.size(), qdbidx == 0, fill_l, fill_r, fill_t,
+                           nl, NC, nstep, q->stall_col};
+    }
     q->stall_col = -1;
-    int64_t cap = std::max<int64_t>(4096 + 16 * (int64_t)nw, q->cand_hint);
+    // room for sixteen reportable cells per column (384 bytes), so that a
+    // window holding a homolog is not scanned twice
+    int64_t columns = 0;
+    for (const trq::Win &x : wl) columns += x.j0 - x.i0 + 1;
+    int64_t cap = std::max<int64_t>(4096 + 16 * columns, q->cand_hint);
     cudaEvent_t ev0, ev1;
     TRQ_TRY(cudaEventCreate(&ev0));
     TRQ_TRY(cudaEventCreate(&ev1));
@@ -1024,9 +1108,15 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
         TRQ_TRY(cudaMemsetAsync(d_queue, 0, sizeof(int) * 2, st));
         TRQ_TRY(cudaMemsetAsync(d_nc, 0, sizeof(unsigned long long), st));
         TRQ_TRY(cudaEventRecord(ev0, st));
-        kfn<<<(unsigned)grid, trq::THREADS, smem, st>>>(tab, d_win, nw, d_dsq, d_decks, deck_stride, cutoff, d_queue,
-                                                       d_c, cap, d_nc, d_res, d_queue + 1);
-        TRQ_TRY(cudaGetLastError());
+        if (diag) {
+            dgp.cand = d_c;
+            dgp.cap = cap;
+            TRQ_TRY(trqd::launch(dgp, (int)grid, warps, st));
+        } else {
+            kfn<<<(unsigned)grid, trq::THREADS, smem, st>>>(tab, d_win, nw, d_dsq, d_decks, deck_stride, cutoff,
+                                                           d_queue, d_c, cap, d_nc, d_res, d_queue + 1);
+            TRQ_TRY(cudaGetLastError());
+        }
         TRQ_TRY(cudaEventRecord(ev1, st));
         unsigned long long nc = 0;
         int kerr = 0;
