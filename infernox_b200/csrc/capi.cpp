@@ -20,6 +20,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <thread>
 #include <vector>
@@ -567,12 +568,9 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     auto chunk_for = [&](int64_t cols) -> int64_t {
         int64_t chunk = ws->chunk;
         if (chunk <= 0 && diag) {
-            // about four pieces per CTA and none shorter than 4W (the warm-up
-            // costs W/2 columns); with too few columns for that, one piece
-            // per CTA, down to W
+            // one piece per CTA, but none shorter than W (the warm-up costs
+            // W/2 columns)
             chunk = std::max<int64_t>((cols + max_ctas - 1) / max_ctas, W);
-            chunk = std::min<int64_t>(chunk, 4 * (int64_t)W);
-            chunk = std::max<int64_t>(chunk, cols / (4 * (int64_t)max_ctas));
             chunk = std::min<int64_t>(chunk, 32768);
         } else if (chunk <= 0 && small_batch) {
             chunk = (cols + max_ctas - 1) / max_ctas;
@@ -587,7 +585,36 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         }
         return chunk;
     };
-    const int64_t batch_chunk = chunk_for(total_cols);
+    int64_t batch_chunk = chunk_for(total_cols);
+    if (diag && ws->chunk <= 0 && !plain) {
+        // Pieces of one to eight per CTA: the length whose longest-first
+        // schedule ends first.  A piece costs its columns, warm-up included,
+        // and about 128 more for the skew of its warps and the empty spans of
+        // its first columns.  (120 uneven windows, M = 379: 466 pieces of 592
+        // columns took 1.6 turns of the 296 CTAs.)
+        double best = 0;
+        int64_t pick = batch_chunk;
+        for (int per = 1; per <= 8; per++) {
+            const int64_t ch = std::min<int64_t>(
+                32768, std::max<int64_t>((total_cols + (int64_t)per * max_ctas - 1) / ((int64_t)per * max_ctas), W));
+            std::vector<int64_t> cost;
+            for (const WinDesc &w : wins)
+                for (int64_t r0 = w.i0; r0 <= w.j0; r0 += ch)
+                    cost.push_back(std::min<int64_t>(w.j0, r0 + ch - 1) - std::max<int64_t>(w.i0, r0 - (W - 1)) + 129);
+            std::sort(cost.begin(), cost.end(), std::greater<int64_t>());
+            std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> ends;
+            int64_t last = 0;
+            for (int64_t x : cost) {
+                int64_t at = 0;
+                if ((int64_t)ends.size() >= max_ctas) at = ends.top(), ends.pop();
+                ends.push(at + x);
+                last = std::max(last, at + x);
+            }
+            if (per == 1 || (double)last < best) best = (double)last, pick = ch;
+            if (ch == W) break;
+        }
+        batch_chunk = pick;
+    }
     for (size_t wi = 0; wi < wins.size(); wi++) {
         const WinDesc &w = wins[wi];
         win_first.push_back(items.size());
@@ -658,6 +685,11 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     }
     int ctas = (int)std::min<int64_t>(((int64_t)items.size() + best_l - 1) / best_l, max_ctas);
     if (diag) {
+        // Warps close together run the same node's code: with every SM full
+        // the instruction cache decides (296 windows of 512: 32 ms at a slack
+        // of 2, 49 at 8), with idle SMs the handshake does (one window of 256:
+        // 10.2 ms at 2, 8.8 at 8).
+        dgp.slack = (int64_t)items.size() >= (int64_t)ws->sm_count * best_c / 2 ? 2 : DG_XCH;
         // the regions stay within half of the free device memory
         size_t freeb = 0, totalb = 0;
         CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
@@ -669,6 +701,7 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         dgp.region = ws->d_diag;
         dgp.next_item = ws->d_counters;
         dgp.cand_count = ws->d_counters + 1;
+        dgp.error = ws->d_counters + 2;
     } else if (!sweep && !deck_smem) {
         // global decks of large models: keep them within half of the free device memory
         size_t freeb = 0, totalb = 0;
@@ -721,7 +754,7 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     };
     size_t ncand = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        CUDA_TRY(cudaMemsetAsync(ws->d_counters, 0, 2 * sizeof(int), ws->stream));
+        CUDA_TRY(cudaMemsetAsync(ws->d_counters, 0, 3 * sizeof(int), ws->stream));
         CUDA_TRY(cudaEventRecord(ws->ev0, ws->stream));
         if (plain) {
             // one launch per window over its own pieces: the per-window comparator
@@ -741,9 +774,13 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
             ws->stats.kernel_launches += 1;
         }
         CUDA_TRY(cudaEventRecord(ws->ev1, ws->stream));
-        CUDA_TRY(cudaMemcpyAsync(ws->h_counters, ws->d_counters, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+        CUDA_TRY(cudaMemcpyAsync(ws->h_counters, ws->d_counters, 3 * sizeof(int), cudaMemcpyDeviceToHost,
                                  ws->stream));
         CUDA_TRY(cudaStreamSynchronize(ws->stream));
+        if (ws->h_counters[2]) {
+            set_error("scan kernel: a wait between warps timed out");
+            return CMGPU_ETIMEOUT;
+        }
         float ms = 0;
         cudaEventElapsedTime(&ms, ws->ev0, ws->ev1);
         ws->stats.kernel_ms += ms;

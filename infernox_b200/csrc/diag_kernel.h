@@ -18,12 +18,18 @@
 
 namespace cmx {
 
-constexpr int DG_CHUNK = 16;                        // spans per phase
+constexpr int DG_CHUNK = 16;                        // spans per step
 constexpr int DG_MAX_WARPS = 16;                    // warps per CTA
 constexpr int DG_COLS = 32 * DG_MAX_WARPS;          // columns per group, at most
 constexpr int DG_PITCH = DG_COLS + 32;              // one row of a node buffer: halo column at 31
 constexpr int DG_SLOTS = 4;                         // split states of a node, at most
 constexpr int DG_ROW = DG_SLOTS * DG_PITCH;         // words per span of a node buffer
+
+constexpr int DG_XCH = 8;                           // steps a warp may be ahead of its right neighbour, at most
+constexpr int DG_STAGE = 4;                         // spans staged at a time
+// words staged per warp: two stages of four split states with a halo and the
+// begin row (three or more where the next node has fewer split states)
+constexpr int DG_STG = 2 * DG_STAGE * (4 * 36 + 32);
 
 // One node, in the order the kernel runs them (last node first; END nodes
 // are constants and have no entry).
@@ -65,6 +71,7 @@ struct DgParams {
     const DgNode *nodes;
     int nnodes;
     const uint32_t *tsc, *endsc, *esc, *el_sca, *bsv;
+    int slack;                   // steps a warp may be ahead of its right neighbour
     int W, ring_cols, ring_len;  // ring_len: residues kept per CTA (power of two)
     int root_dn, root_dxcap;
     int inside, local, begin_key, prefilter, do_null3;
@@ -75,7 +82,7 @@ struct DgParams {
     const uint8_t *dsq;
     const WorkItem *items;
     int nitems, item_base;
-    int *next_item;
+    int *next_item, *error;
     Cand *cands;
     int cand_cap;
     int *cand_count;
