@@ -10,12 +10,21 @@
 // every state of a level depends only on finished levels and itself.  A level
 // is one phase of the CTA: its tasks are spread round-robin over the threads,
 // a task being
-//   * one band row (v, jp) for every state except IR -- its cells d run in
-//     order in one thread, which is exactly what IL's self-transition (cell
-//     d-1 of the same row) needs;
-//   * one diagonal i = j-d+1 for IR states -- IR's self-transition reads
-//     cell (j-1, d-1), the previous cell of the same diagonal, so the thread
-//     walks the diagonal's rows in order.
+//   * one cell for every state but the inserts: neighbouring threads take
+//     neighbouring cells of a band row;
+//   * one chain for an insert state -- IL's self-transition reads cell d-1 of
+//     the same row, so a thread walks a row; IR's reads (j-1, d-1), so a
+//     thread walks a diagonal.  The previous value stays in a register and
+//     the other children of the next cell are loaded before this one is
+//     folded.  (Planes of the truncated scans that have no self-transition
+//     are cells like the others.)
+// A batch of a few hundred envelopes is bound by the latency of one envelope,
+// not by throughput, so the cells of a state run side by side and the CTA
+// takes more threads the fewer envelopes there are.  Measured on one B200 (500
+// envelopes of W = 148, M = 379, bands of +-20, Inside): 7.25 ms with one warp
+// per envelope and one band row per thread, 3.3 here; truncated CYK, 200
+// envelopes: 14.5 ms before, 5.1 here.  What bounds it: the serial chain of an
+// insert state's band row, one of about 120 such levels after the other.
 // Every cell folds its children in the reference's order (children in
 // ascending offset, bifurcation splits k ascending) starting from the local
 // end value, then adds its emission and clamps at IMPOSSIBLE, so the float
@@ -76,10 +85,8 @@ void hb_free(HbDev *h) {
 
 namespace hb {
 
-// threads per envelope CTA: one warp.  A dependency level rarely holds more
-// than a few dozen band rows, a one-warp barrier is cheap, and sixteen
-// envelopes share an SM (measured: 32 threads beat 64 by 20-34 %)
-constexpr int HB_THREADS = 32;
+// threads per envelope CTA, at most (hb_threads picks)
+constexpr int HB_THREADS = 256;
 
 struct Env {
     int64_t alpha_off;  // first cell of this envelope's matrix
@@ -91,9 +98,11 @@ struct Env {
     int32_t pad;
 };
 
-struct State {
-    int32_t jmin, jmax, row0, ntask;  // row0: first Row of state v within its envelope
+struct alignas(16) State {  // loaded in 16-byte words
+    int32_t jmin, jmax, row0, ntask;     // row0: first Row of state v within its envelope; ntask: chains of an
+                                         // insert state, rows of the others
     int32_t ilo, hmn_min, hmx_max, pad;  // IR: first diagonal, band extremes
+    int32_t wide, nj, pad1, pad2;        // widest row, rows
 };
 
 struct Row {  // 8 bytes: band rows dominate the per-call copy
@@ -225,7 +234,34 @@ __device__ void bif_row(const Tables &t, const State *st, const Row *rows, float
     }
 }
 
-// IR state v, diagonal i: cells (j, j-i+1) in row order.
+// One cell d of that row.
+template <bool INS>
+__device__ void bif_cell(const Tables &t, const State *st, const Row *rows, float *alpha, int v, int jp, int d) {
+    const State sv = st[v];
+    const int j = sv.jmin + jp;
+    const Row rv = rows[sv.row0 + jp];
+    const float endsc = t.endsc[v];
+    const bool has_end = endsc > -9.999e35f;
+    const int y = t.cfirst[v], z = t.cnum[v];
+    const State sy = st[y], sz = st[z];
+    const bool inz = j >= sz.jmin && j <= sz.jmax;
+    Row rz{0, 1, 0};
+    if (inz) rz = rows[sz.row0 + j - sz.jmin];
+    const int jpy = j - sy.jmin;
+    const int kn = max(max(j - sy.jmax, rz.hmn), 0), kx = min(jpy, rz.hmx);
+    const int zx = rz.roff - rz.hmn;  // alpha[zx + k] = right child cell k
+    float cur = has_end ? __fadd_rn(__fmul_rn(t.el_selfsc, (float)d), endsc) : IMPOSSIBLE;
+    if (inz)
+#pragma unroll 4
+        for (int k = kn; k <= kx; k++) {
+            const Row ry = rows[sy.row0 + jpy - k];
+            if (k >= d - ry.hmx && k <= d - ry.hmn)
+                cur = comb<INS>(t.flog, cur, __fadd_rn(alpha[ry.roff + (d - ry.hmn - k)], alpha[zx + k]));
+        }
+    alpha[rv.roff - rv.hmn + d] = cur;
+}
+
+// IR state v, diagonal i, cell by cell (many envelopes: fewer registers).
 template <bool INS>
 __device__ void ir_diag(const Tables &t, const State *st, const Row *rows, float *alpha, const uint8_t *dsq, int v,
                         int i) {
@@ -238,13 +274,143 @@ __device__ void ir_diag(const Tables &t, const State *st, const Row *rows, float
     }
 }
 
+// The children of one cell of an insert chain, but for the state itself.
+struct Others {
+    float x[MAXC];
+    int have;  // bit yo: child yo has the cell
+};
+
+// Row jp of an IL state: cells d in order, the self-transition from a register.
 template <bool INS>
-__global__ void __launch_bounds__(HB_THREADS, 16) hb_kernel(Tables t, const Env *__restrict__ envs, int nenv,
+__device__ void il_chain(const Tables &t, const State *st, const Row *rows, float *alpha, const uint8_t *dsq, int v,
+                         int jp) {
+    const State sv = st[v];
+    const int j = sv.jmin + jp;
+    const Row rv = rows[sv.row0 + jp];
+    if (rv.hmn > rv.hmx) return;
+    const float endsc = t.endsc[v];
+    const bool has_end = endsc > -9.999e35f;
+    const int ny = t.cnum[v], y0 = t.cfirst[v], o0 = y0 == v ? 1 : 0;  // child 0 is the state itself
+    int cx[MAXC], clo[MAXC], chi[MAXC];
+    float ct[MAXC];
+#pragma unroll
+    for (int yo = 0; yo < MAXC; yo++) {
+        clo[yo] = 1;
+        chi[yo] = 0;
+        cx[yo] = 0;
+        ct[yo] = 0.0f;
+        if (yo < ny) {
+            ct[yo] = t.tsc[v * MAXC + yo];
+            const State sy = st[y0 + yo];
+            if (yo >= o0 && j >= sy.jmin && j <= sy.jmax) {
+                const Row ry = rows[sy.row0 + j - sy.jmin];
+                cx[yo] = ry.roff - ry.hmn - 1;  // alpha[cx + d] = child cell d - 1
+                clo[yo] = ry.hmn + 1;
+                chi[yo] = ry.hmx + 1;
+            }
+        }
+    }
+    const float *oesc = t.oesc + (size_t)v * ESC;
+    auto load = [&](int d, Others &o, float &e) {
+        o.have = 0;
+        e = 0.0f;
+        if (d > rv.hmx) return;
+#pragma unroll
+        for (int yo = 0; yo < MAXC; yo++)
+            if (d >= clo[yo] && d <= chi[yo]) {
+                o.x[yo] = alpha[cx[yo] + d];
+                o.have |= 1 << yo;
+            }
+        e = oesc[dsq[j - d + 1]];
+    };
+    float *out = alpha + (rv.roff - rv.hmn);
+    Others o, on;
+    float e, en, self = 0.0f;
+    load(rv.hmn, o, e);
+    for (int d = rv.hmn; d <= rv.hmx; d++) {
+        load(d + 1, on, en);
+        float cur = has_end ? __fadd_rn(__fmul_rn(t.el_selfsc, (float)max(d - 1, 0)), endsc) : IMPOSSIBLE;
+        if (o0 && d > rv.hmn) cur = comb<INS>(t.flog, cur, __fadd_rn(self, ct[0]));
+#pragma unroll
+        for (int yo = 0; yo < MAXC; yo++)
+            if (o.have >> yo & 1) cur = comb<INS>(t.flog, cur, __fadd_rn(o.x[yo], ct[yo]));
+        cur = __fadd_rn(cur, e);
+        if (cur < IMPOSSIBLE) cur = IMPOSSIBLE;
+        out[d] = self = cur;
+        o = on;
+        e = en;
+    }
+}
+
+// IR state v, diagonal i: cells (j, j-i+1) in row order, the self-transition
+// (j-1, d-1) from a register.
+template <bool INS>
+__device__ void ir_chain(const Tables &t, const State *st, const Row *rows, float *alpha, const uint8_t *dsq, int v,
+                         int i) {
+    const State sv = st[v];
+    const int jlo = max(sv.jmin, i + sv.hmn_min - 1), jhi = min(sv.jmax, i + sv.hmx_max - 1);
+    const float endsc = t.endsc[v];
+    const bool has_end = endsc > -9.999e35f;
+    const int ny = t.cnum[v], y0 = t.cfirst[v], o0 = y0 == v ? 1 : 0;  // child 0 is the state itself
+    State sy[MAXC];
+    float ct[MAXC];
+#pragma unroll
+    for (int yo = 0; yo < MAXC; yo++) {
+        ct[yo] = yo < ny ? t.tsc[v * MAXC + yo] : 0.0f;
+        if (yo >= o0 && yo < ny) sy[yo] = st[y0 + yo];
+    }
+    const float *oesc = t.oesc + (size_t)v * ESC;
+    auto load = [&](int j, Others &o, float &e, Row &rv) {
+        o.have = 0;
+        e = 0.0f;
+        rv = Row{0, 1, 0};
+        if (j > jhi) return;
+        rv = rows[sv.row0 + j - sv.jmin];
+        const int d = j - i;  // the children's span d - 1
+#pragma unroll
+        for (int yo = 0; yo < MAXC; yo++)
+            if (yo >= o0 && yo < ny && j - 1 >= sy[yo].jmin && j - 1 <= sy[yo].jmax) {
+                const Row ry = rows[sy[yo].row0 + j - 1 - sy[yo].jmin];
+                if (d >= ry.hmn && d <= ry.hmx) {
+                    o.x[yo] = alpha[ry.roff + d - ry.hmn];
+                    o.have |= 1 << yo;
+                }
+            }
+        e = oesc[dsq[j]];
+    };
+    Others o, on;
+    float e, en, self = 0.0f;
+    Row rv, rn;
+    bool prev = false;  // the state holds (j-1, d-1)
+    load(jlo, o, e, rv);
+    for (int j = jlo; j <= jhi; j++) {
+        load(j + 1, on, en, rn);
+        const int d = j - i + 1;
+        if (d >= rv.hmn && d <= rv.hmx) {
+            float cur = has_end ? __fadd_rn(__fmul_rn(t.el_selfsc, (float)max(d - 1, 0)), endsc) : IMPOSSIBLE;
+            if (o0 && prev) cur = comb<INS>(t.flog, cur, __fadd_rn(self, ct[0]));
+#pragma unroll
+            for (int yo = 0; yo < MAXC; yo++)
+                if (o.have >> yo & 1) cur = comb<INS>(t.flog, cur, __fadd_rn(o.x[yo], ct[yo]));
+            cur = __fadd_rn(cur, e);
+            if (cur < IMPOSSIBLE) cur = IMPOSSIBLE;
+            alpha[rv.roff + d - rv.hmn] = self = cur;
+            prev = true;
+        } else {
+            prev = false;
+        }
+        o = on;
+        e = en;
+        rv = rn;
+    }
+}
+
+template <bool INS, bool ROWS>
+__global__ void __launch_bounds__(ROWS ? 32 : HB_THREADS, ROWS ? 16 : 2) hb_kernel(Tables t, const Env *__restrict__ envs, int nenv,
                                                  const State *__restrict__ states, const Row *__restrict__ rows_all,
                                                  float *alpha_all, const uint8_t *__restrict__ dsq_all, int report,
                                                  Cand *cands, int64_t cand_cap, unsigned long long *ncand, Out *out) {
     __shared__ float s_v[HB_THREADS];
-    __shared__ int s_j[HB_THREADS];
     __shared__ int s_envi, s_envj, s_nc;
     const int tid = threadIdx.x, nt = blockDim.x;
     for (int e = blockIdx.x; e < nenv; e += gridDim.x) {
@@ -257,19 +423,29 @@ __global__ void __launch_bounds__(HB_THREADS, 16) hb_kernel(Tables t, const Env 
             int base = 0;
             for (int q = t.lev_start[lev]; q < t.lev_start[lev + 1]; q++) {
                 const int v = t.lev_states[q];
-                const int n = st[v].ntask, stt = t.sttype[v];
+                const int stt = t.sttype[v], wide = ROWS ? 1 : st[v].wide;
+                const int n = stt == IR_ST || (!ROWS && stt == IL_ST) ? st[v].ntask : st[v].nj * wide;
                 // this thread's tasks: base + task = tid (mod nt)
-                for (int task = ((tid - base) % nt + nt) % nt; task < n; task += nt) {
-                    if (stt == IR_ST)
-                        ir_diag<INS>(t, st, rows, alpha, dsq, v, st[v].ilo + task);
-                    else if (stt == B_ST)
-                        bif_row<INS>(t, st, rows, alpha, v, task);
-                    else {
-                        const Row r = rows[st[v].row0 + task];
-                        if (r.hmn <= r.hmx) row_cells<INS>(t, st, rows, alpha, dsq, v, stt, task, r.hmn, r.hmx);
+                for (int task = (tid + nt - base) & (nt - 1); task < n; task += nt) {
+                    if (stt == IR_ST) {
+                        if (ROWS) ir_diag<INS>(t, st, rows, alpha, dsq, v, st[v].ilo + task);
+                        else ir_chain<INS>(t, st, rows, alpha, dsq, v, st[v].ilo + task);
+                    } else if (!ROWS && stt == IL_ST) {
+                        il_chain<INS>(t, st, rows, alpha, dsq, v, task);
+                    } else {
+                        const int jp = ROWS ? task : task / wide;
+                        const Row r = rows[st[v].row0 + jp];
+                        const int d = r.hmn + task - jp * wide, dx = ROWS ? r.hmx : d;
+                        if (d > r.hmx) continue;
+                        if (stt == B_ST && ROWS)
+                            bif_row<INS>(t, st, rows, alpha, v, jp);
+                        else if (stt == B_ST)
+                            bif_cell<INS>(t, st, rows, alpha, v, jp, d);
+                        else
+                            row_cells<INS>(t, st, rows, alpha, dsq, v, stt, jp, d, dx);
                     }
                 }
-                base += n;
+                base = (base + n) & (nt - 1);
             }
             __syncthreads();
         }
@@ -280,59 +456,71 @@ __global__ void __launch_bounds__(HB_THREADS, 16) hb_kernel(Tables t, const Env 
             s_nc = 0;
         }
         __syncthreads();
-        // vsc_root is the first maximum in (j, d) order: per row the first
-        // strict maximum, per thread (rows ascending) a later row wins only
-        // on a strictly larger value, across threads the smallest j wins ties
+        // one ROOT cell per thread (one row where the tasks are rows): the
+        // local begins in order, each on a strictly larger score; vsc_root is
+        // the largest cell
         float best = IMPOSSIBLE;
-        int bestj = INT_MAX;
         const State s0 = st[0];
-        for (int jp = tid; jp <= s0.jmax - s0.jmin; jp += nt) {
-            const int j = s0.jmin + jp;
+        auto report_cell = [&](int j, int d, float sc) {
+            if (sc > best) best = sc;
+            if (sc >= env.env_cutoff) {
+                atomicMin(&s_envi, j - d + 1);
+                atomicMax(&s_envj, j);
+            }
+            if (report && d >= 1 && sc >= env.cutoff && sc > -9.999e35f) {
+                const unsigned long long slot = atomicAdd(ncand, 1ull);
+                atomicAdd(&s_nc, 1);
+                if ((int64_t)slot < cand_cap) cands[slot] = Cand{e, j, d, sc};
+            }
+        };
+        if (ROWS) {
+            for (int jp = tid; jp < s0.nj; jp += nt) {
+                const int j = s0.jmin + jp;
+                const Row r0 = rows[s0.row0 + jp];
+                const int av = r0.roff - r0.hmn;
+                if (t.local_begin)
+                    for (int b = 0; b < t.nbeg; b++) {
+                        const int y = t.begins[b];
+                        const State sy = st[y];
+                        if (j < sy.jmin || j > sy.jmax) continue;
+                        const Row ry = rows[sy.row0 + j - sy.jmin];
+                        const int dn = max(r0.hmn, ry.hmn), dx = min(r0.hmx, ry.hmx);
+                        const float bsc = t.beginsc[y];
+                        for (int d = dn; d <= dx; d++) {
+                            const float sc = __fadd_rn(alpha[ry.roff + d - ry.hmn], bsc);
+                            if (sc > alpha[av + d]) alpha[av + d] = sc;
+                        }
+                    }
+                for (int d = r0.hmn; d <= r0.hmx; d++) report_cell(j, d, alpha[av + d]);
+            }
+        }
+        for (int task = tid; !ROWS && task < s0.nj * s0.wide; task += nt) {
+            const int jp = task / s0.wide, j = s0.jmin + jp;
             const Row r0 = rows[s0.row0 + jp];
-            const int av = r0.roff - r0.hmn;
-            if (t.local_begin)
+            const int d = r0.hmn + task - jp * s0.wide;
+            if (d > r0.hmx) continue;
+            float sc = alpha[r0.roff - r0.hmn + d];
+            if (t.local_begin) {
+#pragma unroll 4
                 for (int b = 0; b < t.nbeg; b++) {
                     const int y = t.begins[b];
                     const State sy = st[y];
                     if (j < sy.jmin || j > sy.jmax) continue;
                     const Row ry = rows[sy.row0 + j - sy.jmin];
-                    const int dn = max(r0.hmn, ry.hmn), dx = min(r0.hmx, ry.hmx);
-                    const float bsc = t.beginsc[y];
-                    for (int d = dn; d <= dx; d++) {
-                        const float sc = __fadd_rn(alpha[ry.roff + d - ry.hmn], bsc);
-                        if (sc > alpha[av + d]) alpha[av + d] = sc;
-                    }
+                    if (d < ry.hmn || d > ry.hmx) continue;
+                    const float x = __fadd_rn(alpha[ry.roff + d - ry.hmn], t.beginsc[y]);
+                    if (x > sc) sc = x;
                 }
-            float rb = IMPOSSIBLE;
-            for (int d = r0.hmn; d <= r0.hmx; d++) {
-                const float sc = alpha[av + d];
-                if (sc > rb) rb = sc;
-                if (sc >= env.env_cutoff) {
-                    atomicMin(&s_envi, j - d + 1);
-                    atomicMax(&s_envj, j);
-                }
-                if (report && d >= 1 && sc >= env.cutoff && sc > -9.999e35f) {
-                    const unsigned long long slot = atomicAdd(ncand, 1ull);
-                    atomicAdd(&s_nc, 1);
-                    if ((int64_t)slot < cand_cap) cands[slot] = Cand{e, j, d, sc};
-                }
+                alpha[r0.roff - r0.hmn + d] = sc;
             }
-            if (rb > best) {
-                best = rb;
-                bestj = j;
-            }
+            report_cell(j, d, sc);
         }
         s_v[tid] = best;
-        s_j[tid] = bestj;
         __syncthreads();
         if (tid == 0) {
             float bv = IMPOSSIBLE;
-            int bj = INT_MAX;
             for (int q = 0; q < nt; q++)
-                if (s_v[q] > bv || (s_v[q] == bv && s_j[q] < bj)) {
-                    bv = s_v[q];
-                    bj = s_j[q];
-                }
+                if (s_v[q] > bv) bv = s_v[q];
             out[e] = Out{bv, s_envi == INT_MAX ? -1 : s_envi, s_envj == INT_MIN ? -1 : s_envj, s_nc};
         }
         __syncthreads();
@@ -382,8 +570,10 @@ __device__ __forceinline__ int tr_bits(const State *st, int y, const TrTab &tr) 
     return (b & 1) | ((b & 2) && tr.fill_l ? 2 : 0) | ((b & 4) && tr.fill_r ? 4 : 0) | ((b & 8) && tr.fill_t ? 8 : 0);
 }
 
-// Cells dlo..dhi of row jp of a non-bifurcation state v (all four planes).
-template <bool INS>
+// Cells dlo..dhi of row jp of a non-bifurcation state v: all four planes, or
+// (ALL false) of an insert state the planes without a self-transition: R of
+// IL, L of IR.
+template <bool INS, bool ALL>
 __device__ void tr_row(const Tables &t, const TrTab &tr, const State *st, const Row *rows, float *PJ, float *PL,
                        float *PR, float *PT, const uint8_t *dsq, int v, int stt, int jp, int dlo, int dhi) {
     const State sv = st[v];
@@ -434,7 +624,7 @@ __device__ void tr_row(const Tables &t, const TrTab &tr, const State *st, const 
         float J = dj ? init(d, sd) : IMPOSSIBLE, L = dl ? init(d, sdl) : IMPOSSIBLE, R = dr ? init(d, sdr) : IMPOSSIBLE;
         if (stt == ML_ST || stt == IL_ST) {
             const float e = oesc[dsq[j - d + 1]];
-            if (dj || dl) {
+            if ((ALL || stt == ML_ST) && (dj || dl)) {
 #pragma unroll
                 for (int yo = 0; yo < MAXC; yo++) {
                     const bool djy = cbits[yo] & 1, dly = cbits[yo] & 2;
@@ -468,7 +658,7 @@ __device__ void tr_row(const Tables &t, const TrTab &tr, const State *st, const 
             }
         } else if (stt == MR_ST || stt == IR_ST) {
             const float e = oesc[xj];
-            if (dj || dr) {
+            if ((ALL || stt == MR_ST) && (dj || dr)) {
 #pragma unroll
                 for (int yo = 0; yo < MAXC; yo++) {
                     const bool djy = cbits[yo] & 1, dry = cbits[yo] & 4;
@@ -550,17 +740,113 @@ __device__ void tr_row(const Tables &t, const TrTab &tr, const State *st, const 
                 }
             }
         }
-        PJ[c] = J;
-        PL[c] = L;
-        PR[c] = R;
+        if (ALL || (stt != IL_ST && stt != IR_ST)) PJ[c] = J;
+        if (ALL || stt != IL_ST) PL[c] = L;
+        if (ALL || stt != IR_ST) PR[c] = R;
         PT[c] = IMPOSSIBLE;
     }
 }
 
-// Row jp of a bifurcation state v (all four planes).
+// The children of one cell of an insert chain, but for the state itself: two
+// planes (J and L of an IL state, J and R of an IR state).
+struct TrOthers {
+    float x[MAXC], z[MAXC];
+    int have;  // bit yo: child yo has the cell
+};
+
+// Chain `task` of an insert state: planes J and L of a row of an IL state, J
+// and R of a diagonal of an IR state, the self-transition from registers.
+template <bool INS, bool IL>
+__device__ void tr_chain(const Tables &t, const TrTab &tr, const State *st, const Row *rows, float *PJ, float *PZ,
+                         const uint8_t *dsq, int v, int task) {
+    const State sv = st[v];
+    const int vb = tr_bits(st, v, tr), zbit = IL ? 2 : 4;
+    const bool dj = vb & 1, dz = vb & zbit;
+    const float endsc = t.endsc[v];
+    const bool has_end = endsc > IMPOSSIBLE + 1.0f;
+    const int ny = t.cnum[v], y0 = t.cfirst[v], o0 = y0 == v ? 1 : 0;  // child 0 is the state itself
+    State sy[MAXC];
+    float ct[MAXC];
+    int bits[MAXC];
+#pragma unroll
+    for (int yo = 0; yo < MAXC; yo++) {
+        ct[yo] = yo < ny ? t.tsc[v * MAXC + yo] : 0.0f;
+        bits[yo] = yo < ny ? tr_bits(st, y0 + yo, tr) : 0;
+        if (yo >= o0 && yo < ny) sy[yo] = st[y0 + yo];
+    }
+    const float *oesc = t.oesc + (size_t)v * ESC;
+    // IL: row j, cells d ascending; IR: diagonal i, rows j ascending
+    const int j0 = sv.jmin + task, i0 = sv.ilo + task;
+    Row r0{0, 1, 0};
+    if (IL) r0 = rows[sv.row0 + task];
+    const int first = IL ? r0.hmn : max(sv.jmin, i0 + sv.hmn_min - 1);
+    const int last = IL ? r0.hmx : min(sv.jmax, i0 + sv.hmx_max - 1);
+    auto load = [&](int s, TrOthers &o, float &e, Row &rv) {
+        o.have = 0;
+        e = 0.0f;
+        rv = IL ? r0 : Row{0, 1, 0};
+        if (s > last) return;
+        const int j = IL ? j0 : s, d = IL ? s : s - i0 + 1, jy = IL ? j : j - 1;
+        if (!IL) rv = rows[sv.row0 + j - sv.jmin];
+#pragma unroll
+        for (int yo = 0; yo < MAXC; yo++)
+            if (yo >= o0 && yo < ny && (bits[yo] & (1 | zbit)) && jy >= sy[yo].jmin && jy <= sy[yo].jmax) {
+                const Row ry = rows[sy[yo].row0 + jy - sy[yo].jmin];
+                if (d - 1 >= ry.hmn && d - 1 <= ry.hmx) {
+                    const int cy = ry.roff + d - 1 - ry.hmn;
+                    if (bits[yo] & 1) o.x[yo] = PJ[cy];
+                    if (bits[yo] & zbit) o.z[yo] = PZ[cy];
+                    o.have |= 1 << yo;
+                }
+            }
+        e = oesc[IL ? dsq[j - d + 1] : dsq[j]];
+    };
+    TrOthers o, on;
+    float e, en, selfj = 0.0f, selfz = 0.0f;
+    Row rv, rn;
+    bool prev = false;
+    load(first, o, e, rv);
+    for (int s = first; s <= last; s++) {
+        load(s + 1, on, en, rn);
+        const int d = IL ? s : s - i0 + 1;
+        if (d >= rv.hmn && d <= rv.hmx) {
+            const float a = has_end && d >= 1 ? __fadd_rn(__fmul_rn(t.el_selfsc, (float)(d - 1)), endsc) : IMPOSSIBLE;
+            float J = dj ? a : IMPOSSIBLE, Z = dz ? a : IMPOSSIBLE;
+            if (o0 && prev) {
+                if (dj) J = comb<INS>(t.flog, J, __fadd_rn(selfj, ct[0]));
+                if (dz) Z = comb<INS>(t.flog, Z, __fadd_rn(selfz, ct[0]));
+            }
+#pragma unroll
+            for (int yo = 0; yo < MAXC; yo++)
+                if (o.have >> yo & 1) {
+                    if (dj && (bits[yo] & 1)) J = comb<INS>(t.flog, J, __fadd_rn(o.x[yo], ct[yo]));
+                    if (dz && (bits[yo] & zbit)) Z = comb<INS>(t.flog, Z, __fadd_rn(o.z[yo], ct[yo]));
+                }
+            if (dj) {
+                J = __fadd_rn(J, e);
+                if (J < IMPOSSIBLE) J = IMPOSSIBLE;
+            }
+            if (dz) {
+                Z = d >= 2 ? __fadd_rn(Z, e) : e;
+                if (Z < IMPOSSIBLE) Z = IMPOSSIBLE;
+            }
+            const int c = rv.roff + d - rv.hmn;
+            PJ[c] = selfj = J;
+            PZ[c] = selfz = Z;
+            prev = true;
+        } else {
+            prev = false;
+        }
+        o = on;
+        e = en;
+        rv = rn;
+    }
+}
+
+// Cell d of row jp of a bifurcation state v (all four planes).
 template <bool INS>
-__device__ void tr_bif_row(const Tables &t, const TrTab &tr, const State *st, const Row *rows, float *PJ, float *PL,
-                           float *PR, float *PT, int v, int jp) {
+__device__ void tr_bif_cell(const Tables &t, const TrTab &tr, const State *st, const Row *rows, float *PJ, float *PL,
+                            float *PR, float *PT, int v, int jp, int d) {
     const State sv = st[v];
     const int j = sv.jmin + jp;
     const Row rv = rows[sv.row0 + jp];
@@ -576,7 +862,7 @@ __device__ void tr_bif_row(const Tables &t, const TrTab &tr, const State *st, co
     const CRow rz = crow(st, rows, z, j), ry = crow(st, rows, y, j);
     const int jpy = j - sy.jmin;
     const int kn = max(max(j - sy.jmax, rz.hmn), 0), kx = min(jpy, rz.hmx);
-    for (int d = rv.hmn; d <= rv.hmx; d++) {
+    {
         const float e0 = has_end ? __fadd_rn(__fmul_rn(t.el_selfsc, (float)d), endsc) : IMPOSSIBLE;
         float J = dj ? e0 : IMPOSSIBLE, L = dl ? e0 : IMPOSSIBLE, R = dr ? e0 : IMPOSSIBLE, T = IMPOSSIBLE;
         if (rz.ok)
@@ -607,8 +893,8 @@ __device__ void tr_bif_row(const Tables &t, const TrTab &tr, const State *st, co
     }
 }
 
-template <bool INS>
-__global__ void __launch_bounds__(HB_THREADS, 16) tr_kernel(Tables t, TrTab tr, const Env *__restrict__ envs, int nenv,
+template <bool INS, bool ROWS>
+__global__ void __launch_bounds__(ROWS ? 32 : HB_THREADS, ROWS ? 16 : 1) tr_kernel(Tables t, TrTab tr, const Env *__restrict__ envs, int nenv,
                                                  const State *__restrict__ states, const Row *__restrict__ rows_all,
                                                  float *planes, int64_t plane_stride, const uint8_t *__restrict__ dsq_all,
                                                  int report, TrCand *cands, int64_t cand_cap,
@@ -628,26 +914,47 @@ __global__ void __launch_bounds__(HB_THREADS, 16) tr_kernel(Tables t, TrTab tr, 
             for (int q = t.lev_start[lev]; q < t.lev_start[lev + 1]; q++) {
                 const int v = t.lev_states[q];
                 if (v == 0) continue;  // ROOT: truncated begins in the root pass
-                const int n = st[v].ntask, stt = t.sttype[v];
-                for (int task = ((tid - base) % nt + nt) % nt; task < n; task += nt) {
-                    if (stt == IR_ST) {
-                        const State sv = st[v];
-                        const int i = sv.ilo + task;
-                        const int jlo = max(sv.jmin, i + sv.hmn_min - 1), jhi = min(sv.jmax, i + sv.hmx_max - 1);
-                        for (int j = jlo; j <= jhi; j++) {
-                            const int d = j - i + 1;
-                            const Row rv = rows[sv.row0 + j - sv.jmin];
-                            if (d >= rv.hmn && d <= rv.hmx)
-                                tr_row<INS>(t, tr, st, rows, PJ, PL, PR, PT, dsq, v, IR_ST, j - sv.jmin, d, d);
+                const int stt = t.sttype[v], wide = st[v].wide, ncell = st[v].nj * wide;
+                if (ROWS) {
+                    const int n = stt == IR_ST ? st[v].ntask : st[v].nj;
+                    for (int task = (tid + nt - base) & (nt - 1); task < n; task += nt) {
+                        if (stt == IR_ST) {
+                            const State sv = st[v];
+                            const int i = sv.ilo + task;
+                            const int jlo = max(sv.jmin, i + sv.hmn_min - 1), jhi = min(sv.jmax, i + sv.hmx_max - 1);
+                            for (int j = jlo; j <= jhi; j++) {
+                                const int d = j - i + 1;
+                                const Row rv = rows[sv.row0 + j - sv.jmin];
+                                if (d >= rv.hmn && d <= rv.hmx)
+                                    tr_row<INS, true>(t, tr, st, rows, PJ, PL, PR, PT, dsq, v, IR_ST, j - sv.jmin, d, d);
+                            }
+                            continue;
                         }
-                    } else if (stt == B_ST) {
-                        tr_bif_row<INS>(t, tr, st, rows, PJ, PL, PR, PT, v, task);
-                    } else {
                         const Row r = rows[st[v].row0 + task];
-                        if (r.hmn <= r.hmx) tr_row<INS>(t, tr, st, rows, PJ, PL, PR, PT, dsq, v, stt, task, r.hmn, r.hmx);
+                        if (stt == B_ST)
+                            for (int x = r.hmn; x <= r.hmx; x++) tr_bif_cell<INS>(t, tr, st, rows, PJ, PL, PR, PT, v, task, x);
+                        else if (r.hmn <= r.hmx)
+                            tr_row<INS, true>(t, tr, st, rows, PJ, PL, PR, PT, dsq, v, stt, task, r.hmn, r.hmx);
                     }
+                    base = (base + n) & (nt - 1);
+                    continue;
                 }
-                base += n;
+                // chains of an insert state first, then one cell per task
+                const int nchain = stt == IL_ST || stt == IR_ST ? st[v].ntask : 0, n = nchain + ncell;
+                for (int task = (tid + nt - base) & (nt - 1); task < n; task += nt) {
+                    if (task < nchain) {
+                        if (stt == IL_ST) tr_chain<INS, true>(t, tr, st, rows, PJ, PL, dsq, v, task);
+                        else tr_chain<INS, false>(t, tr, st, rows, PJ, PR, dsq, v, task);
+                        continue;
+                    }
+                    const int jp = (task - nchain) / wide;
+                    const Row r = rows[st[v].row0 + jp];
+                    const int d = r.hmn + (task - nchain) - jp * wide;
+                    if (d > r.hmx) continue;
+                    if (stt == B_ST) tr_bif_cell<INS>(t, tr, st, rows, PJ, PL, PR, PT, v, jp, d);
+                    else tr_row<INS, false>(t, tr, st, rows, PJ, PL, PR, PT, dsq, v, stt, jp, d, d);
+                }
+                base = (base + n) & (nt - 1);
             }
             __syncthreads();
         }
@@ -903,6 +1210,19 @@ int hb_prepare(cmgpu_model *m, HbDev **out) {
     return CMGPU_OK;
 }
 
+// Threads per envelope CTA.  With few envelopes an SM has room for every cell
+// of a level at once; with many the GPU is full anyway, and one warp per
+// envelope with a row per thread does the least work.  Kernel ms (256 / 128
+// threads / 32 by rows): HB Inside, 200 envelopes 2.3 / 2.9 / 6.2, 500 4.4 /
+// 3.3 / 7.2, 1,000 - / 6.2 / 8.3, 2,000 14.8 / 11.4 / 9.7; truncated CYK (twice
+// the registers), 40 envelopes 3.0 / 4.5 / 11, 200 5.3 / 5.1 / 14.5, 1,000 - /
+// 19.1 / 22.3, 2,000 37.3 / 35.6 / 32.1.
+int hb_threads(int device, int nenv, bool truncated) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return nenv > 10 * sms ? 32 : nenv > (truncated ? 1 : 2) * sms ? 128 : 256;
+}
+
 int sdelta_h(int st) { return st == MP_ST ? 2 : (st == ML_ST || st == MR_ST || st == IL_ST || st == IR_ST) ? 1 : 0; }
 
 // rows of one envelope's bands (the sum of its states' j-ranges)
@@ -931,7 +1251,7 @@ int64_t fill_envelope(const HostCM &c, const cmgpu_hb_task &tk, int64_t dsq_len,
     int32_t nrow = 0;
     for (int v = 0; v < M; v++) {
         const int st = c.sttype[v], sd = sdelta_h(st);
-        hb::State s{b.jmin[v], b.jmax[v], nrow, 0, 0, INT_MAX, INT_MIN, 0};
+        hb::State s{b.jmin[v], b.jmax[v], nrow, 0, 0, INT_MAX, INT_MIN, 0, 0, 0, 0, 0};
         const int nj = b.jmax[v] >= b.jmin[v] ? b.jmax[v] - b.jmin[v] + 1 : 0;
         const int32_t *hmn_v = b.hdmin + b.hd_off[v], *hmx_v = b.hdmax + b.hd_off[v];
         int ilo = INT_MAX, ihi = INT_MIN;
@@ -958,7 +1278,10 @@ int64_t fill_envelope(const HostCM &c, const cmgpu_hb_task &tk, int64_t dsq_len,
                 return -1;
             }
             rows[nrow++] = hb::Row{(int32_t)ncells, (int16_t)hmn, (int16_t)hmx};
-            if (hmx >= hmn) ncells += hmx - hmn + 1;
+            if (hmx >= hmn) {
+                ncells += hmx - hmn + 1;
+                s.wide = std::max(s.wide, hmx - hmn + 1);
+            }
         }
         if (ncells > INT32_MAX) {
             err = "HMM-banded scan: more than 2^31 band cells in one envelope";
@@ -970,6 +1293,7 @@ int64_t fill_envelope(const HostCM &c, const cmgpu_hb_task &tk, int64_t dsq_len,
         } else {
             s.ntask = nj;
         }
+        s.nj = nj;
         states[v] = s;
     }
     return ncells;
@@ -1071,6 +1395,7 @@ int hb_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, int repor
     hb::Tables t{h->sttype, h->cfirst, h->cnum, h->lev_start, h->lev_states, h->begins, h->tsc, h->oesc,
                  h->endsc, h->beginsc, h->flog, m->cm.view.el_selfsc, h->nlev, h->nbeg,
                  (int)((m->cm.view.flags >> 10) & 1u)};
+    const int threads = hb_threads(m->device, n, false);
     int64_t cap = report ? std::max<int64_t>(4096 + 16 * (int64_t)n, h->cand_hint) : 0;
     cudaEvent_t ev0, ev1;
     HB_TRY(cudaEventCreate(&ev0));
@@ -1085,12 +1410,10 @@ int hb_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, int repor
         }
         HB_TRY(cudaMemsetAsync(d_nc, 0, sizeof(unsigned long long), st));
         HB_TRY(cudaEventRecord(ev0, st));
-        if (semiring == CMGPU_INSIDE_F32)
-            hb::hb_kernel<true><<<n, hb::HB_THREADS, 0, st>>>(t, d_env, n, d_st, d_rows, d_alpha, d_dsq, report, d_c, cap, d_nc,
-                                                   d_out);
-        else
-            hb::hb_kernel<false><<<n, hb::HB_THREADS, 0, st>>>(t, d_env, n, d_st, d_rows, d_alpha, d_dsq, report, d_c, cap, d_nc,
-                                                    d_out);
+        const bool ins = semiring == CMGPU_INSIDE_F32;
+        auto kern = threads > 32 ? (ins ? hb::hb_kernel<true, false> : hb::hb_kernel<false, false>)
+                                 : (ins ? hb::hb_kernel<true, true> : hb::hb_kernel<false, true>);
+        kern<<<n, threads, 0, st>>>(t, d_env, n, d_st, d_rows, d_alpha, d_dsq, report, d_c, cap, d_nc, d_out);
         HB_TRY(cudaGetLastError());
         HB_TRY(cudaEventRecord(ev1, st));
         unsigned long long nc = 0;
@@ -1251,6 +1574,7 @@ int tr_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, const hb:
     hb::Tables t{h->sttype, h->cfirst, h->cnum, h->lev_start, h->lev_states, h->begins, h->tsc, h->oesc,
                  h->endsc, h->beginsc, h->flog, m->cm.view.el_selfsc, h->nlev, h->nbeg,
                  (int)((m->cm.view.flags >> 10) & 1u)};
+    const int threads = hb_threads(m->device, n, true);
     int64_t cap = report ? std::max<int64_t>(4096 + 16 * (int64_t)n, h->tr_cand_hint) : 0;
     cudaEvent_t ev0, ev1;
     HB_TRY(cudaEventCreate(&ev0));
@@ -1265,12 +1589,10 @@ int tr_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, const hb:
         }
         HB_TRY(cudaMemsetAsync(d_nc, 0, sizeof(unsigned long long), st));
         HB_TRY(cudaEventRecord(ev0, st));
-        if (semiring == CMGPU_INSIDE_F32)
-            hb::tr_kernel<true><<<n, hb::HB_THREADS, 0, st>>>(t, trt, d_env, n, d_st, d_rows, d_planes, cells, d_dsq, report, d_c,
-                                                   cap, d_nc, d_out);
-        else
-            hb::tr_kernel<false><<<n, hb::HB_THREADS, 0, st>>>(t, trt, d_env, n, d_st, d_rows, d_planes, cells, d_dsq, report,
-                                                    d_c, cap, d_nc, d_out);
+        const bool ins = semiring == CMGPU_INSIDE_F32;
+        auto kern = threads > 32 ? (ins ? hb::tr_kernel<true, false> : hb::tr_kernel<false, false>)
+                                 : (ins ? hb::tr_kernel<true, true> : hb::tr_kernel<false, true>);
+        kern<<<n, threads, 0, st>>>(t, trt, d_env, n, d_st, d_rows, d_planes, cells, d_dsq, report, d_c, cap, d_nc, d_out);
         HB_TRY(cudaGetLastError());
         HB_TRY(cudaEventRecord(ev1, st));
         unsigned long long nc = 0;
