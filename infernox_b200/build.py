@@ -11,7 +11,7 @@ LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libcmscan_gpu.so")
 
 SOURCES = ["trq_diag.cu", "qdb_scan.cu", "diag_scan.cu", "diag_plan.cpp", "sweep_scan.cu", "capi.cpp", "cm_prep.cpp", "qdb_plan.cpp", "noalloc.cu", "p7_vit.cu", "p7_msv.cu", "hb_scan.cu", "trq_scan.cu", "calibrate.cpp", "p7_fwd.cu"]
-HEADERS = ["devbuf.h", "trq_diag.h", "diag_kernel.h", "plan_util.h", "report_device.cuh", "trunc_report.h", "cm_internal.h", "qdb_plan.h", "qdb_kernel.h", "model_internal.h",
+HEADERS = ["replay.h", "devbuf.h", "trq_diag.h", "diag_kernel.h", "plan_util.h", "report_device.cuh", "trunc_report.h", "cm_internal.h", "qdb_plan.h", "qdb_kernel.h", "model_internal.h",
            "semiring.cuh", "sweep_plan.h", "sweep_kernel.h"]
 
 NVCC_FLAGS = [

@@ -17,7 +17,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <queue>
@@ -30,6 +29,7 @@
 #include "model_internal.h"
 #include "qdb_kernel.h"
 #include "qdb_plan.h"
+#include "replay.h"
 #include "diag_kernel.h"
 #include "sweep_kernel.h"
 
@@ -246,33 +246,11 @@ static inline float raw_bits(int semiring, uint32_t raw) {
     return f;
 }
 
-// remove_overlaps_greedy (src/cp9.rs:6544-6574): hits sorted by score
-// (descending, stable) then start; a hit is removed when it overlaps an
-// earlier hit that was kept.  The kept hits are disjoint, so they are held
-// in a map ordered by start: the only kept hit that can overlap [i, j] is the
-// one with the largest start <= j, and it overlaps when its end >= i.  Same
-// result as the pairwise scan, in O(n log n).
-static void remove_overlaps(std::vector<cmgpu_hit> &h) {
-    std::stable_sort(h.begin(), h.end(), [](const cmgpu_hit &a, const cmgpu_hit &b) {
-        if (a.score != b.score) return a.score > b.score;
-        return a.i < b.i;
-    });
-    std::map<int32_t, int32_t> kept;  // start -> end
-    size_t o = 0;
-    for (size_t x = 0; x < h.size(); x++) {
-        auto it = kept.upper_bound(h[x].j);
-        if (it != kept.begin() && std::prev(it)->second >= h[x].i) continue;
-        kept.emplace(h[x].i, h[x].j);
-        h[o++] = h[x];
-    }
-    h.resize(o);
-}
-
-// Replays report_hits_greedily for one window from its candidate cells
-// (sorted by j, d).  frame = window frame (host), needed for null3.
-void report_window(const cmgpu_model *m, int semiring, const Cand *c, size_t n, const uint8_t *frame,
-                          int32_t i0, float cutoff, int do_null3, std::vector<cmgpu_hit> &out) {
-    std::vector<cmgpu_hit> tmp;
+// Replays report_hits_greedily for columns of one window from their candidate
+// cells (sorted by j, d); the report of a column does not depend on the
+// others.  frame = window frame (host), needed for null3.
+static void report_columns(const cmgpu_model *m, int semiring, const Cand *c, size_t n, const uint8_t *frame,
+                           int32_t i0, float cutoff, int do_null3, std::vector<cmgpu_hit> &tmp) {
     // prefix counts of canonical residues over the candidates' span
     std::vector<int32_t> pre;
     int32_t lo = 0;
@@ -323,6 +301,13 @@ void report_window(const cmgpu_model *m, int semiring, const Cand *c, size_t n, 
             }
         }
     }
+}
+
+// The whole window: every column's report, then the overlap removal.
+void report_window(const cmgpu_model *m, int semiring, const Cand *c, size_t n, const uint8_t *frame,
+                   int32_t i0, float cutoff, int do_null3, std::vector<cmgpu_hit> &out) {
+    std::vector<cmgpu_hit> tmp;
+    report_columns(m, semiring, c, n, frame, i0, cutoff, do_null3, tmp);
     remove_overlaps(tmp);
     out.insert(out.end(), tmp.begin(), tmp.end());
 }
@@ -665,7 +650,10 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     // Room for one reportable cell per four columns (4 bytes of device memory
     // per residue): batches with homologs in a tenth of their sequences stay
     // well inside it, so the scan is not repeated with a larger buffer.
-    const size_t cand_cap = std::max<size_t>({ws->cands_cap, (size_t)1 << 16, (size_t)(total_cols / 4)});
+    // cmcalibrate's scan has no cutoff: in a glocal model a dozen cells of a
+    // column exceed all shorter ones.
+    const size_t per_cand = calib ? (size_t)total_cols * 18 : (size_t)(total_cols / 4);
+    const size_t cand_cap = std::max<size_t>({ws->cands_cap, (size_t)1 << 16, per_cand});
     if ((rc = ensure_dev(&ws->d_cands, &ws->cands_cap, cand_cap))) return rc;
     if (!diag && !sweep && !deck_smem && (int64_t)items.size() < best_l) {
         // fewer work items than lanes: no deck for lanes that would stay idle
@@ -843,11 +831,11 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
         }
         std::sort(f, l, jd_less);
     };
-    {
+    on_cores(items.size(), ncand, 1 << 14, [&](size_t x) {
         std::vector<size_t> at;
         std::vector<Cand> tmp;
-        for (size_t x = 0; x < items.size(); x++) order_item((size_t)rank[x], items[x], at, tmp);
-    }
+        if (start[(size_t)rank[x] + 1] > start[(size_t)rank[x]]) order_item((size_t)rank[x], items[x], at, tmp);
+    });
     if (cells_out) {
         *cells_out = cs;
         return CMGPU_OK;
@@ -879,25 +867,34 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
             }
         }
     }
-    // report_hits_greedily + overlap removal per window: windows are
-    // independent, so they are replayed on the host's cores
-    auto replay = [&](size_t r) {
-        const Range &g = ranges[r];
-        report_window(m, semiring, cs.data() + g.b, g.e - g.b, g.frame, wins[g.win].i0, cutoff, do_null3,
-                      hits_per_win[g.win]);
+    // report_hits_greedily on pieces of whole columns, then the overlap
+    // removal of each window, on the host's cores
+    struct Piece {
+        size_t range, b, e;
     };
-    const size_t nthr = std::min<size_t>(ranges.size(), std::max(1u, std::thread::hardware_concurrency()));
-    if (nthr <= 1 || cs.size() < (1u << 16)) {
-        for (size_t r = 0; r < ranges.size(); r++) replay(r);
-    } else {
-        std::atomic<size_t> next{0};
-        std::vector<std::thread> pool;
-        for (size_t t = 0; t < nthr; t++)
-            pool.emplace_back([&]() {
-                for (size_t r; (r = next.fetch_add(1)) < ranges.size();) replay(r);
-            });
-        for (auto &th : pool) th.join();
+    constexpr size_t PIECE = 1 << 13;  // cells
+    std::vector<Piece> pieces;
+    std::vector<size_t> first(ranges.size() + 1, 0);
+    for (size_t r = 0; r < ranges.size(); r++) {
+        for (size_t k = ranges[r].b; k < ranges[r].e;) {
+            size_t e = std::min(k + PIECE, ranges[r].e);
+            while (e < ranges[r].e && cs[e].j == cs[e - 1].j) e++;
+            pieces.push_back(Piece{r, k, e});
+            k = e;
+        }
+        first[r + 1] = pieces.size();
     }
+    std::vector<std::vector<cmgpu_hit>> part(pieces.size());
+    on_cores(pieces.size(), cs.size(), 2 * PIECE, [&](size_t q) {
+        const Range &g = ranges[pieces[q].range];
+        report_columns(m, semiring, cs.data() + pieces[q].b, pieces[q].e - pieces[q].b, g.frame, wins[g.win].i0, cutoff,
+                       do_null3, part[q]);
+    });
+    on_cores(ranges.size(), cs.size(), 2 * PIECE, [&](size_t r) {
+        std::vector<cmgpu_hit> &h = hits_per_win[ranges[r].win];
+        for (size_t q = first[r]; q < first[r + 1]; q++) h.insert(h.end(), part[q].begin(), part[q].end());
+        remove_overlaps(h);
+    });
     (void)dsq_len;
     return CMGPU_OK;
 }

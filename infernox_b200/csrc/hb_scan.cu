@@ -46,6 +46,7 @@
 
 #include "devbuf.h"
 #include "model_internal.h"
+#include "replay.h"
 #include "trunc_report.h"
 
 namespace cmx {
@@ -60,6 +61,7 @@ struct HbDev {
     int32_t last_launches = 0;
     DevArena arena;          // per-call device buffers (tables, matrix, results), reused
     PinnedBuf st_pin, row_pin;  // per-call host band tables, staged in pinned memory
+    PinnedBuf cand_pin;         // a launch's reportable cells
     int64_t cand_hint = 0;   // reportable cells the last call needed
     int64_t tr_cand_hint = 0;  // the same for the truncated scans
 };
@@ -69,6 +71,7 @@ void hb_free(HbDev *h) {
     h->arena.release();
     h->st_pin.release();
     h->row_pin.release();
+    h->cand_pin.release();
     cudaFree(h->sttype);
     cudaFree(h->cfirst);
     cudaFree(h->cnum);
@@ -1128,18 +1131,8 @@ void tr_report(const cmgpu_model *m, const TrCtx &cx, const hb::TrCand *c, size_
             }
         }
     }
-    std::stable_sort(tmp.begin(), tmp.end(), [](const cmgpu_tr_hit &a, const cmgpu_tr_hit &b) {
-        if (a.score != b.score) return a.score > b.score;
-        return a.i < b.i;
-    });
-    std::vector<char> removed(tmp.size(), 0);
-    for (size_t a = 0; a < tmp.size(); a++) {
-        if (removed[a]) continue;
-        for (size_t b = a + 1; b < tmp.size(); b++)
-            if (!removed[b] && !(tmp[b].j < tmp[a].i) && !(tmp[a].j < tmp[b].i)) removed[b] = 1;
-    }
-    for (size_t a = 0; a < tmp.size(); a++)
-        if (!removed[a]) out.push_back(tmp[a]);
+    remove_overlaps(tmp);
+    out.insert(out.end(), tmp.begin(), tmp.end());
 }
 
 namespace {
@@ -1430,29 +1423,31 @@ int hb_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, int repor
             h->cand_hint = cap;
             continue;
         }
-        std::vector<hb::Cand> hc((size_t)nc);
+        hb::Cand *hc = h->cand_pin.get<hb::Cand>((size_t)std::max<unsigned long long>(nc, 1));
+        if (!hc) {
+            cudaEventDestroy(ev0);
+            cudaEventDestroy(ev1);
+            set_error("HMM-banded scan: pinned host allocation failed");
+            return CMGPU_ENOMEM;
+        }
         if (nc) {
-            HB_TRY(cudaMemcpyAsync(hc.data(), d_c, sizeof(hb::Cand) * (size_t)nc, cudaMemcpyDeviceToHost, st));
+            HB_TRY(cudaMemcpyAsync(hc, d_c, sizeof(hb::Cand) * (size_t)nc, cudaMemcpyDeviceToHost, st));
             HB_TRY(cudaStreamSynchronize(st));
         }
-        std::sort(hc.begin(), hc.end(), [](const hb::Cand &a, const hb::Cand &b) {
-            if (a.env != b.env) return a.env < b.env;
-            if (a.j != b.j) return a.j < b.j;
-            return a.d < b.d;
-        });
-        size_t q = 0;
-        for (int e = 0; e < n; e++) {
+        std::vector<hb::Cand> cells_jd;
+        std::vector<std::vector<cmgpu_hit>> per(n);
+        replay_cells(hc, (size_t)nc, (size_t)n, cells_jd, [&](size_t e, const hb::Cand *c0, size_t k) {
             const cmgpu_hb_task &tk = tasks[e0 + e];
+            if (report) hb_report(m, c0, k, dsq_all + tk.dsq_offset, tk.i0, tk.cutoff, do_null3, per[e]);
+        });
+        for (int e = 0; e < n; e++) {
             cmgpu_hb_result &r = results[e0 + e];
             r.vsc_root = outv[e].vsc;
             r.envi = outv[e].envi;
             r.envj = outv[e].envj;
             r.hit_first = (int64_t)hits.size();
-            size_t q1 = q;
-            while (q1 < hc.size() && hc[q1].env == e) q1++;
-            if (report) hb_report(m, hc.data() + q, q1 - q, dsq_all + tk.dsq_offset, tk.i0, tk.cutoff, do_null3, hits);
-            r.nhits = (int32_t)((int64_t)hits.size() - r.hit_first);
-            q = q1;
+            hits.insert(hits.end(), per[e].begin(), per[e].end());
+            r.nhits = (int32_t)per[e].size();
         }
         break;
     }
@@ -1609,32 +1604,33 @@ int tr_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, const hb:
             h->tr_cand_hint = cap;
             continue;
         }
-        std::vector<hb::TrCand> hc((size_t)nc);
+        hb::TrCand *hc = h->cand_pin.get<hb::TrCand>((size_t)std::max<unsigned long long>(nc, 1));
+        if (!hc) {
+            cudaEventDestroy(ev0);
+            cudaEventDestroy(ev1);
+            set_error("truncated HMM-banded scan: pinned host allocation failed");
+            return CMGPU_ENOMEM;
+        }
         if (nc) {
-            HB_TRY(cudaMemcpyAsync(hc.data(), d_c, sizeof(hb::TrCand) * (size_t)nc, cudaMemcpyDeviceToHost, st));
+            HB_TRY(cudaMemcpyAsync(hc, d_c, sizeof(hb::TrCand) * (size_t)nc, cudaMemcpyDeviceToHost, st));
             HB_TRY(cudaStreamSynchronize(st));
         }
-        std::sort(hc.begin(), hc.end(), [](const hb::TrCand &a, const hb::TrCand &b) {
-            if (a.env != b.env) return a.env < b.env;
-            if (a.j != b.j) return a.j < b.j;
-            return a.d < b.d;
-        });
-        size_t q = 0;
-        for (int e = 0; e < n; e++) {
+        std::vector<hb::TrCand> cells_jd;
+        std::vector<std::vector<cmgpu_tr_hit>> per(n);
+        replay_cells(hc, (size_t)nc, (size_t)n, cells_jd, [&](size_t e, const hb::TrCand *c0, size_t k) {
             const cmgpu_tr_task &tk = tasks[e0 + e];
+            if (report)
+                tr_report(m, cx, c0, k, dsq_all + tk.dsq_offset, tk.i0, tk.j0, tk.cutoff, do_null3, per[e]);
+        });
+        for (int e = 0; e < n; e++) {
             cmgpu_tr_result &r = results[e0 + e];
             r.vsc_root = outv[e].vsc;
             r.vmode = outv[e].vmode;
             r.envi = outv[e].envi;
             r.envj = outv[e].envj;
             r.hit_first = (int64_t)hits.size();
-            size_t q1 = q;
-            while (q1 < hc.size() && hc[q1].env == e) q1++;
-            if (report)
-                tr_report(m, cx, hc.data() + q, q1 - q, dsq_all + tk.dsq_offset, tk.i0, tk.j0, tk.cutoff, do_null3,
-                          hits);
-            r.nhits = (int32_t)((int64_t)hits.size() - r.hit_first);
-            q = q1;
+            hits.insert(hits.end(), per[e].begin(), per[e].end());
+            r.nhits = (int32_t)per[e].size();
         }
         break;
     }

@@ -61,6 +61,7 @@
 #include "devbuf.h"
 #include "model_internal.h"
 #include "plan_util.h"
+#include "replay.h"
 #include "trq_diag.h"
 #include "trunc_report.h"
 
@@ -78,6 +79,7 @@ struct TrqDev {
     int nlev = 0, nbegl = 0;
     DevArena arena;
     int64_t cand_hint = 0;
+    PinnedBuf cand_pin;  // the call's reportable cells
     double last_ms = 0;
     int64_t last_cells = 0;
     int32_t last_launches = 0;
@@ -88,6 +90,7 @@ struct TrqDev {
 void trq_free(TrqDev *t) {
     if (!t) return;
     t->arena.release();
+    t->cand_pin.release();
     cudaFree(t->sttype);
     cudaFree(t->kind);
     cudaFree(t->cfirst);
@@ -1096,7 +1099,8 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     cudaEvent_t ev0, ev1;
     TRQ_TRY(cudaEventCreate(&ev0));
     TRQ_TRY(cudaEventCreate(&ev1));
-    std::vector<hb::TrCand> hc;
+    hb::TrCand *hc = nullptr;
+    size_t nhc = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
         hb::TrCand *d_c = nullptr;
         if (ar.get(14, &d_c, sizeof(hb::TrCand) * (size_t)cap)) {
@@ -1138,9 +1142,15 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
             q->cand_hint = cap;
             continue;
         }
-        hc.resize((size_t)nc);
-        if (nc)
-            TRQ_TRY(cudaMemcpyAsync(hc.data(), d_c, sizeof(hb::TrCand) * (size_t)nc, cudaMemcpyDeviceToHost, st));
+        nhc = (size_t)nc;
+        hc = q->cand_pin.get<hb::TrCand>(std::max<size_t>(nhc, 1));
+        if (!hc) {
+            cudaEventDestroy(ev0);
+            cudaEventDestroy(ev1);
+            set_error("truncated QDB scan: pinned host allocation failed");
+            return CMGPU_ENOMEM;
+        }
+        if (nc) TRQ_TRY(cudaMemcpyAsync(hc, d_c, sizeof(hb::TrCand) * nhc, cudaMemcpyDeviceToHost, st));
         break;
     }
     cudaEventDestroy(ev0);
@@ -1148,27 +1158,24 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     std::vector<trq::Res> rv(nwin);
     TRQ_TRY(cudaMemcpyAsync(rv.data(), d_res, sizeof(trq::Res) * nwin, cudaMemcpyDeviceToHost, st));
     TRQ_TRY(cudaStreamSynchronize(st));
-    std::sort(hc.begin(), hc.end(), [](const hb::TrCand &a, const hb::TrCand &b) {
-        if (a.env != b.env) return a.env < b.env;
-        if (a.j != b.j) return a.j < b.j;
-        return a.d < b.d;
-    });
     const TrCtx cx{tt, pass_idx, tt->local};
-    size_t p = 0;
-    for (int32_t e = 0; e < nwin; e++) {
+    std::vector<hb::TrCand> cells_jd;
+    std::vector<std::vector<cmgpu_tr_hit>> per(nwin);
+    replay_cells(hc, nhc, (size_t)nwin, cells_jd, [&](size_t e, const hb::TrCand *c0, size_t n) {
         const cmgpu_window &wd = wins[e];
+        if (wd.j0 >= wd.i0)
+            tr_report(m, cx, c0, n, dsq_all + wd.dsq_offset, wd.i0, wd.j0, cutoff, do_null3, per[e]);
+    });
+    for (int32_t e = 0; e < nwin; e++) {
         cmgpu_trq_result &r = results[e];
         r.hit_first = (int64_t)hits.size();
-        size_t p1 = p;
-        while (p1 < hc.size() && hc[p1].env == e) p1++;
-        if (wd.j0 >= wd.i0) {
+        if (wins[e].j0 >= wins[e].i0) {
             r.vsc_root = rv[e].vsc;
             r.vmode = rv[e].vmode;
             r.bsc_full = rv[e].bsc_full;
-            tr_report(m, cx, hc.data() + p, p1 - p, dsq_all + wd.dsq_offset, wd.i0, wd.j0, cutoff, do_null3, hits);
         }
-        r.nhits = (int32_t)((int64_t)hits.size() - r.hit_first);
-        p = p1;
+        hits.insert(hits.end(), per[e].begin(), per[e].end());
+        r.nhits = (int32_t)per[e].size();
     }
     return CMGPU_OK;
 }
