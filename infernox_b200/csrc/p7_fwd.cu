@@ -51,7 +51,8 @@ namespace cmx {
 void set_error(const std::string &msg);
 int f1_msv_windows_vec(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, int64_t dsq_len,
                        const cmgpu_window *chunks, int32_t nchunk, double f1, int64_t cmw,
-                       std::vector<cmgpu_f1_window> &wins);
+                       std::vector<cmgpu_f1_window> &wins, int share_device = -1,
+                       const uint8_t **d_residues = nullptr);
 }
 using cmx::set_error;
 
@@ -509,8 +510,10 @@ int check_windows(const char *who, const uint8_t *dsq_all, int64_t dsq_len, cons
 }
 
 // Forward pieces (totscale, xC) and bias rows of every window, on the device
-// (either output may be null).  The residue buffer is copied once.
-int score_windows(const cmgpu_fwd_filter *f, cudaStream_t st, const uint8_t *dsq_all, int64_t dsq_len,
+// (either output may be null).  The residue buffer is copied once, or not at
+// all where a stage before has it on the device already (`d_have`, written on
+// `st` and left alone until this returns).
+int score_windows(const cmgpu_fwd_filter *f, cudaStream_t st, const uint8_t *dsq_all, int64_t dsq_len, const uint8_t *d_have,
                   const cmgpu_window *wins, int32_t nwin, const uint8_t *want_fwd, std::vector<float> *fwd_ts,
                   std::vector<float> *fwd_xc, std::vector<float> *bias_rows) {
     cmgpu_fwd_filter *mf = const_cast<cmgpu_fwd_filter *>(f);
@@ -538,13 +541,13 @@ int score_windows(const cmgpu_fwd_filter *f, cudaStream_t st, const uint8_t *dsq
             const cmgpu_window &w = wins[k];
             fw[(size_t)nf + k] = {w.dsq_offset + w.i0, std::max(0, w.j0 - w.i0 + 1), 0};
         }
-    uint8_t *d_dsq = nullptr;
+    uint8_t *d_up = nullptr;
     cmx::dev::FwdWin *d_w = nullptr;
     float2 *d_out = nullptr;
     float *d_rows = nullptr;
     int *d_next = nullptr;
     cudaError_t e = cudaSuccess;
-    if ((e = mf->arena.get(0, &d_dsq, (size_t)dsq_len)) != cudaSuccess ||
+    if ((!d_have && (e = mf->arena.get(0, &d_up, (size_t)dsq_len)) != cudaSuccess) ||
         (e = mf->arena.get(1, &d_w, sizeof(cmx::dev::FwdWin) * fw.size())) != cudaSuccess ||
         (e = mf->arena.get(2, &d_out, sizeof(float2) * std::max(nf, 1))) != cudaSuccess ||
         (e = mf->arena.get(3, &d_rows, sizeof(float) * (size_t)nwin)) != cudaSuccess ||
@@ -552,7 +555,8 @@ int score_windows(const cmgpu_fwd_filter *f, cudaStream_t st, const uint8_t *dsq
         set_error(std::string("cmgpu_fwd: ") + cudaGetErrorString(e));
         return CMGPU_ENOMEM;
     }
-    FWD_TRY(cudaMemcpyAsync(d_dsq, dsq_all, (size_t)dsq_len, cudaMemcpyHostToDevice, st));
+    if (!d_have) FWD_TRY(cudaMemcpyAsync(d_up, dsq_all, (size_t)dsq_len, cudaMemcpyHostToDevice, st));
+    const uint8_t *d_dsq = d_have ? d_have : d_up;
     FWD_TRY(cudaMemcpyAsync(d_w, fw.data(), sizeof(cmx::dev::FwdWin) * fw.size(), cudaMemcpyHostToDevice, st));
     FWD_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), st));
     // launch shape: as many groups of four as fit, tables in shared memory
@@ -711,7 +715,7 @@ extern "C" int cmgpu_fwd_score_batch(const cmgpu_fwd_filter *f, void *stream, co
     int rc = check_windows("cmgpu_fwd_score_batch", dsq_all, dsq_len, wins, nwin);
     if (rc) return rc;
     std::vector<float> ts, xc, rows;
-    rc = score_windows(f, (cudaStream_t)stream, dsq_all, dsq_len, wins, nwin, nullptr, fwd_scores ? &ts : nullptr,
+    rc = score_windows(f, (cudaStream_t)stream, dsq_all, dsq_len, nullptr, wins, nwin, nullptr, fwd_scores ? &ts : nullptr,
                        fwd_scores ? &xc : nullptr, bias_scores ? &rows : nullptr);
     if (rc) return rc;
     for (int32_t k = 0; k < nwin; k++) {
@@ -782,8 +786,10 @@ extern "C" int cmgpu_f3_filter(const cmgpu_fwd_filter *ff, const cmgpu_msv_filte
     int32_t dev_launches = 0;
     // windows: SSV (F1) or deterministic 2*maxW tiles (src/cm_pipeline.rs:1890-1915)
     std::vector<cmgpu_f1_window> w1;
+    const uint8_t *d_have = nullptr;  // the residues on the device, from the SSV stage
     if (cfg->do_msv) {
-        rc = cmx::f1_msv_windows_vec(mf, st, dsq_all, dsq_len, chunks, nchunk, cfg->f1, cfg->cmw, w1);
+        rc = cmx::f1_msv_windows_vec(mf, st, dsq_all, dsq_len, chunks, nchunk, cfg->f1, cfg->cmw, w1,
+                                     ff->device, &d_have);
         if (rc) return rc;
         double ms = 0;
         int32_t l = 0;
@@ -823,7 +829,7 @@ extern "C" int cmgpu_f3_filter(const cmgpu_fwd_filter *ff, const cmgpu_msv_filte
     };
     // F3 and F3b scores in one pass when no earlier stage gates the windows
     if (nw > 0 && (need_bias || (cfg->do_fwd && !gated))) {
-        rc = score_windows(ff, st, dsq_all, dsq_len, bw.data(), nw, nullptr,
+        rc = score_windows(ff, st, dsq_all, dsq_len, d_have, bw.data(), nw, nullptr,
                            cfg->do_fwd && !gated ? &ts : nullptr, cfg->do_fwd && !gated ? &xc : nullptr,
                            need_bias ? &rows : nullptr);
         if (rc) return rc;
@@ -891,7 +897,7 @@ extern "C" int cmgpu_f3_filter(const cmgpu_fwd_filter *ff, const cmgpu_msv_filte
     }
     // F3 Forward on the windows that reach it, when earlier stages gated them
     if (cfg->do_fwd && gated && nw > 0) {
-        rc = score_windows(ff, st, dsq_all, dsq_len, bw.data(), nw, reach.data(), &ts, &xc, nullptr);
+        rc = score_windows(ff, st, dsq_all, dsq_len, d_have, bw.data(), nw, reach.data(), &ts, &xc, nullptr);
         if (rc) return rc;
         add_fwd_stats();
     }

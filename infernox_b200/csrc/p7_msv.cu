@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) msv_score_kernel(const uint32_t *__restri
 
 struct SsvSeg {
     int64_t off;  // buffer index of local residue 1 minus 1
-    int32_t r0, r1, w0, pad;
+    int32_t r0, r1, w0, chunk;
 };
 
 struct SsvCand {
@@ -376,12 +376,24 @@ __global__ void __launch_bounds__(256) ssv_scan_kernel(const uint32_t *__restric
     }
 }
 
-// Sequential trigger logic of ssv_diagonals over one chunk per warp.
+// Sequential trigger logic of ssv_diagonals.  A trigger's state -- the row z it
+// resets the scan at and the row the walk resumes at -- reaches at most 2M rows
+// beyond the candidate it came from: the extension adds at most M rows, and
+// from M-1 rows after the reset the rows are the free-running ones again.  So
+// a candidate with no other one in the 2M rows before it (a clean one) starts
+// afresh, and each warp takes the run from the first clean candidate of its
+// segment to the first clean candidate of a later segment.  So every candidate
+// has one warp, which writes the window it triggers (or none, n = 0) to the
+// candidate's own slot and counts it in nraw of the candidate's segment.  What
+// bounds it is the chain of dependent steps of a warp, not memory, so it wants
+// many warps.  (One warp per chunk of 100 kb took 0.8 ms for 9.2 Mb of M = 120; a warp per
+// segment 0.1 ms.)
 template <int R>
 __global__ void __launch_bounds__(128) ssv_replay_kernel(const uint32_t *__restrict__ negc, const uint8_t *__restrict__ rbv,
                                                          int M, int bias, int xbb, int thr, int base, int tjb,
                                                          int tbm, float scale_b, const uint8_t *__restrict__ dsq,
-                                                         const SsvChunk *__restrict__ chunks, int nchunk, int cap,
+                                                         const SsvChunk *__restrict__ chunks,
+                                                         const SsvSeg *__restrict__ segs, int nseg, int cap,
                                                          const SsvCand *__restrict__ cands,
                                                          const int *__restrict__ counts, SsvRaw *raws, int *nraw,
                                                          int *need) {
@@ -390,27 +402,39 @@ __global__ void __launch_bounds__(128) ssv_replay_kernel(const uint32_t *__restr
     __syncthreads();
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const uint32_t bias2 = pack2(bias), xbb2 = pack2(xbb);
-    for (int c = blockIdx.x * nw + (threadIdx.x >> 5); c < nchunk; c += gridDim.x * nw) {
-        const SsvChunk ch = chunks[c];
+    for (int s0 = blockIdx.x * nw + (threadIdx.x >> 5); s0 < nseg; s0 += gridDim.x * nw) {
+        const SsvChunk ch = chunks[segs[s0].chunk];
         const uint8_t *frame = dsq + ch.off;
-        bool bad = false;
-        for (int s = ch.seg_first; s < ch.seg_first + ch.seg_count; s++)
-            if (counts[s] > cap) {
-                bad = true;
-                if (lane == 0) atomicMax(need, counts[s]);
-            }
-        if (bad) {
-            if (lane == 0) nraw[c] = 0;
+        if (counts[s0] > cap) {
+            if (lane == 0) atomicMax(need, counts[s0]);
             continue;
         }
+        // row of the last candidate before this segment, 2M rows back at most
+        int last = INT_MIN / 2;
+        for (int s = s0 - 1; s >= ch.seg_first && segs[s].r1 > segs[s0].r0 - 2 * M; s--)
+            if (counts[s] > 0) {
+                last = counts[s] > cap ? segs[s].r1 : cands[(int64_t)s * cap + counts[s] - 1].row;
+                break;
+            }
         uint32_t w[R];
-        int z = 1, i = 1, hz = -1, hr = 0, nr = 0;
-        SsvRaw *out = raws + (int64_t)ch.seg_first * cap;
-        for (int s = ch.seg_first; s < ch.seg_first + ch.seg_count; s++) {
-            const int cnt = counts[s];
+        int z = 1, i = 1, hz = -1, hr = 0;
+        bool started = false, done = false;
+        for (int s = s0; s < ch.seg_first + ch.seg_count && !done; s++) {
+            const int cnt = min(counts[s], cap);
+            SsvRaw *out = raws + (int64_t)s * cap;
+            int nr = 0;
             for (int ci = 0; ci < cnt; ci++) {
                 const SsvCand cd = cands[(int64_t)s * cap + ci];
                 const int r = cd.row;
+                const bool clean = r - last >= 2 * M;
+                last = r;
+                if (clean && s > s0) {  // the warp of segment s takes over
+                    done = true;
+                    break;
+                }
+                if (!started && !clean) continue;  // the run of an earlier segment
+                started = true;
+                if (lane == 0) out[ci].n = 0;
                 if (r < i) continue;
                 int xe = cd.xe, ek = cd.k;
                 if (z != 1 && r < z + M - 1) {
@@ -487,14 +511,60 @@ __global__ void __launch_bounds__(128) ssv_replay_kernel(const uint32_t *__restr
                 if (lane == 0) {
                     const int end_model = ek + (max_end - r);
                     const float sc = (__fsub_rn((float)(max_sc - tjb), (float)base) / scale_b) - 3.0f;
-                    out[nr] = SsvRaw{tstart, end_model - start + 1, end_model, sc};
+                    out[ci] = SsvRaw{tstart, end_model - start + 1, end_model, sc};
                 }
                 nr++;
                 z = max_end + 1;
                 i = max_end + 1;
             }
+            if (lane == 0 && nr > 0) atomicAdd(&nraw[s], nr);
+            if (!started) break;  // every candidate of the segment belongs to an earlier run
         }
-        if (lane == 0) nraw[c] = nr;
+    }
+}
+
+// Each chunk's windows as one list, in order, at a place of its own in `out`
+// (where[2c] the first, where[2c + 1] how many; `fill` the places given out),
+// so that one copy brings them all to the host.  One block per chunk, a thread
+// per segment.
+__global__ void __launch_bounds__(256) ssv_gather_kernel(const SsvChunk *__restrict__ chunks, int cap,
+                                                         const int *__restrict__ counts, const int *__restrict__ nraw,
+                                                         const SsvRaw *__restrict__ raws, SsvRaw *__restrict__ out,
+                                                         int *where, int *fill) {
+    __shared__ int ws[8], base;
+    const SsvChunk ch = chunks[blockIdx.x];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    int run = 0;
+    for (int pass = 0; pass < 2; pass++) {
+        for (int s0 = 0; s0 < ch.seg_count; s0 += 256) {
+            const int s = ch.seg_first + s0 + threadIdx.x;
+            const int n = s0 + threadIdx.x < ch.seg_count ? nraw[s] : 0;
+            const int incl = warp_incl_sum(n, lane);
+            if (lane == 31) ws[wi] = incl;
+            __syncthreads();
+            int at = run + incl - n;
+            for (int q = 0; q < 8; q++) {
+                if (q < wi) at += ws[q];
+                run += ws[q];
+            }
+            if (pass == 1 && n > 0) {
+                const int cnt = min(counts[s], cap);
+                for (int k = 0; k < cnt; k++) {
+                    const SsvRaw w = raws[(int64_t)s * cap + k];
+                    if (w.n > 0) out[at++] = w;
+                }
+            }
+            __syncthreads();
+        }
+        if (pass == 0) {
+            if (threadIdx.x == 0) {
+                base = atomicAdd(fill, run);
+                where[2 * blockIdx.x] = base;
+                where[2 * blockIdx.x + 1] = run;
+            }
+            __syncthreads();
+            run = base;
+        }
     }
 }
 
@@ -551,7 +621,10 @@ void launch_msv(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *d_dsq
 template <int R>
 void launch_ssv(const cmgpu_msv_filter *f, cudaStream_t st, int xbb, int thr, const uint8_t *d_dsq,
                 const dev::SsvSeg *d_segs, int nseg, const dev::SsvChunk *d_ch, int nch, int cap,
-                dev::SsvCand *d_cands, int *d_counts, dev::SsvRaw *d_raws, int *d_nraw, int *d_need) {
+                dev::SsvCand *d_cands, int *d_counts, dev::SsvRaw *d_raws, dev::SsvRaw *d_out, int *d_info) {
+    // d_info: the candidate slots wanted, the windows found, each segment's
+    // windows, each chunk's place and count
+    int *d_nraw = d_info + 2, *d_where = d_nraw + nseg;
     const size_t smem = (size_t)KP * R * 32 * sizeof(uint32_t);
     cmx::allow_max_dynamic_smem(dev::ssv_scan_kernel<R>);
     const MsvHost &h = f->host;
@@ -559,9 +632,10 @@ void launch_ssv(const cmgpu_msv_filter *f, cudaStream_t st, int xbb, int thr, co
                                                               d_cands, d_counts);
     const size_t rsm = (size_t)(h.M + 1) * KP;
     cmx::allow_max_dynamic_smem(dev::ssv_replay_kernel<R>);
-    dev::ssv_replay_kernel<R><<<(nch + 3) / 4, 128, rsm, st>>>(f->d_negc, f->d_rbv, h.M, h.bias_b, xbb, thr, h.base_b,
-                                                            h.tjb_b, h.tbm_b, h.scale_b, d_dsq, d_ch, nch, cap, d_cands,
-                                                            d_counts, d_raws, d_nraw, d_need);
+    dev::ssv_replay_kernel<R><<<(nseg + 3) / 4, 128, rsm, st>>>(f->d_negc, f->d_rbv, h.M, h.bias_b, xbb, thr, h.base_b,
+                                                             h.tjb_b, h.tbm_b, h.scale_b, d_dsq, d_ch, d_segs, nseg,
+                                                             cap, d_cands, d_counts, d_raws, d_nraw, d_info);
+    dev::ssv_gather_kernel<<<nch, 256, 0, st>>>(d_ch, cap, d_counts, d_nraw, d_raws, d_out, d_where, d_info + 1);
 }
 
 #define DISPATCH_R(R, CALL)                  \
@@ -652,7 +726,7 @@ int ssv_run(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, 
         ch[c] = dev::SsvChunk{off, l, (int32_t)segs.size(), 0, 0};
         for (int64_t r0 = 1; r0 <= l; r0 += seg_len) {
             const int32_t r1 = (int32_t)std::min<int64_t>(l, r0 + seg_len - 1);
-            segs.push_back(dev::SsvSeg{off, (int32_t)r0, r1, (int32_t)std::max<int64_t>(1, r0 - (M - 1)), 0});
+            segs.push_back(dev::SsvSeg{off, (int32_t)r0, r1, (int32_t)std::max<int64_t>(1, r0 - (M - 1)), c});
         }
         ch[c].seg_count = (int32_t)segs.size() - ch[c].seg_first;
     }
@@ -661,13 +735,13 @@ int ssv_run(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, 
     uint8_t *d_dsq;
     dev::SsvSeg *d_segs;
     dev::SsvChunk *d_ch;
-    int *d_counts, *d_nraw, *d_need;
+    int *d_counts, *d_info;
     MSV_ALLOC(0, d_dsq, (size_t)dsq_len);
     MSV_ALLOC(1, d_segs, sizeof(dev::SsvSeg) * nseg);
     MSV_ALLOC(2, d_ch, sizeof(dev::SsvChunk) * nch);
     MSV_ALLOC(3, d_counts, sizeof(int) * nseg);
-    MSV_ALLOC(4, d_nraw, sizeof(int) * nch);
-    MSV_ALLOC(5, d_need, sizeof(int));
+    const size_t ninfo = 2 + (size_t)nseg + 2 * (size_t)nch;
+    MSV_ALLOC(4, d_info, sizeof(int) * ninfo);
     MSV_TRY(cudaMemcpyAsync(d_dsq, dsq_all, (size_t)dsq_len, cudaMemcpyHostToDevice, st));
     MSV_TRY(cudaMemcpyAsync(d_segs, segs.data(), sizeof(dev::SsvSeg) * nseg, cudaMemcpyHostToDevice, st));
     MSV_TRY(cudaMemcpyAsync(d_ch, ch.data(), sizeof(dev::SsvChunk) * nch, cudaMemcpyHostToDevice, st));
@@ -679,45 +753,40 @@ int ssv_run(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, 
     int launches = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
         dev::SsvCand *d_cands;
-        dev::SsvRaw *d_raws;
+        dev::SsvRaw *d_raws, *d_out;
         cudaError_t e;
         if ((e = f->arena.get(6, &d_cands, sizeof(dev::SsvCand) * (size_t)nseg * cap)) != cudaSuccess ||
-            (e = f->arena.get(7, &d_raws, sizeof(dev::SsvRaw) * (size_t)nseg * cap)) != cudaSuccess) {
+            (e = f->arena.get(7, &d_raws, sizeof(dev::SsvRaw) * (size_t)nseg * cap)) != cudaSuccess ||
+            (e = f->arena.get(5, &d_out, sizeof(dev::SsvRaw) * (size_t)nseg * cap)) != cudaSuccess) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             set_error(std::string("msv: device allocation: ") + cudaGetErrorString(e));
             return CMGPU_ENOMEM;
         }
-        MSV_TRY(cudaMemsetAsync(d_need, 0, sizeof(int), st));
+        MSV_TRY(cudaMemsetAsync(d_info, 0, sizeof(int) * (2 + (size_t)nseg), st));
         MSV_TRY(cudaEventRecord(e0, st));
 #define CALL_SSV(RR) \
-    launch_ssv<RR>(f, st, xbb, thr, d_dsq, d_segs, nseg, d_ch, nch, cap, d_cands, d_counts, d_raws, d_nraw, d_need)
+    launch_ssv<RR>(f, st, xbb, thr, d_dsq, d_segs, nseg, d_ch, nch, cap, d_cands, d_counts, d_raws, d_out, d_info)
         DISPATCH_R(f->R, CALL_SSV);
 #undef CALL_SSV
         MSV_TRY(cudaGetLastError());
         MSV_TRY(cudaEventRecord(e1, st));
-        int need = 0;
-        std::vector<int> nraw(nch);
-        MSV_TRY(cudaMemcpyAsync(&need, d_need, sizeof(int), cudaMemcpyDeviceToHost, st));
-        MSV_TRY(cudaMemcpyAsync(nraw.data(), d_nraw, sizeof(int) * nch, cudaMemcpyDeviceToHost, st));
+        std::vector<int> info(2), where(2 * (size_t)nch);
+        MSV_TRY(cudaMemcpyAsync(info.data(), d_info, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+        MSV_TRY(cudaMemcpyAsync(where.data(), d_info + 2 + nseg, sizeof(int) * 2 * nch, cudaMemcpyDeviceToHost, st));
         MSV_TRY(cudaStreamSynchronize(st));
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
         ms_total += ms;
-        launches += 2;
+        launches += 3;
+        const int need = info[0];
         if (need > cap) {
             cap = need + need / 4;
             f->cap_hint = cap;
             continue;
         }
-        // only each chunk's windows come back (they sit at the chunk's first
-        // segment slot), into pinned memory
-        size_t nall = 0;
-        std::vector<size_t> at(nch);
-        for (int32_t c = 0; c < nch; c++) {
-            at[c] = nall;
-            nall += (size_t)std::max(0, nraw[c]);
-        }
+        // only the windows come back, into pinned memory
+        const size_t nall = (size_t)info[1];
         dev::SsvRaw *hr = f->raw_pin.get<dev::SsvRaw>(std::max<size_t>(nall, 1));
         if (!hr) {
             cudaEventDestroy(e0);
@@ -725,14 +794,14 @@ int ssv_run(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, 
             set_error("msv: pinned host allocation failed");
             return CMGPU_ENOMEM;
         }
-        for (int32_t c = 0; c < nch; c++)
-            if (nraw[c] > 0)
-                MSV_TRY(cudaMemcpyAsync(hr + at[c], d_raws + (size_t)ch[c].seg_first * cap,
-                                        sizeof(dev::SsvRaw) * (size_t)nraw[c], cudaMemcpyDeviceToHost, st));
-        MSV_TRY(cudaStreamSynchronize(st));
+        if (nall > 0) {
+            MSV_TRY(cudaMemcpyAsync(hr, d_out, sizeof(dev::SsvRaw) * nall, cudaMemcpyDeviceToHost, st));
+            MSV_TRY(cudaStreamSynchronize(st));
+        }
         for (int32_t c = 0; c < nch; c++) {
-            const dev::SsvRaw *p = hr + at[c];
-            for (int q = 0; q < nraw[c]; q++) raws[c].push_back(RawWin{p[q].n, p[q].length, p[q].k, p[q].score});
+            const dev::SsvRaw *p = hr + where[2 * c];
+            raws[c].reserve(where[2 * c + 1]);
+            for (int q = 0; q < where[2 * c + 1]; q++) raws[c].push_back(RawWin{p[q].n, p[q].length, p[q].k, p[q].score});
         }
         break;
     }
@@ -912,15 +981,24 @@ extern "C" int cmgpu_ssv_diagonals(const cmgpu_msv_filter *f, void *stream, cons
 
 namespace cmx {
 // f1_msv_windows on every chunk into a vector (windows grouped by chunk);
-// the chunks have been checked by the caller.
+// the chunks have been checked by the caller.  *d_residues: where the residues
+// stay on the device until the filter's next call, if that is `share_device`
+// and any were scanned; left alone otherwise.
 int f1_msv_windows_vec(const cmgpu_msv_filter *f, cudaStream_t st, const uint8_t *dsq_all, int64_t dsq_len,
                        const cmgpu_window *chunks, int32_t nchunk, double f1, int64_t cmw,
-                       std::vector<cmgpu_f1_window> &wins) {
+                       std::vector<cmgpu_f1_window> &wins, int share_device, const uint8_t **d_residues) {
     MSV_TRY(cudaSetDevice(f->device));
     std::vector<std::vector<RawWin>> raws;
     int rc = ssv_run(f, st, dsq_all, dsq_len, chunks, nchunk, f1, raws);
     if (rc) return rc;
     wins.clear();
+    if (d_residues && share_device == f->device && std::any_of(raws.begin(), raws.end(), [](const auto &r) {
+            return !r.empty();
+        })) {
+        uint8_t *d;
+        MSV_ALLOC(0, d, (size_t)dsq_len);  // ssv_run's buffer: no larger one is made
+        *d_residues = d;
+    }
     for (int32_t c = 0; c < nchunk; c++)
         extend_merge_split(f->host, raws[c], std::max(0, chunks[c].j0 - chunks[c].i0 + 1), cmw, c, wins);
     return CMGPU_OK;
@@ -939,7 +1017,7 @@ extern "C" int cmgpu_f1_msv_windows(const cmgpu_msv_filter *f, void *stream, con
     int rc = check_windows("cmgpu_f1_msv_windows", dsq_all, dsq_len, chunks, nchunk);
     if (rc) return rc;
     std::vector<cmgpu_f1_window> wins;
-    rc = cmx::f1_msv_windows_vec(f, (cudaStream_t)stream, dsq_all, dsq_len, chunks, nchunk, f1, cmw, wins);
+    rc = cmx::f1_msv_windows_vec(f, (cudaStream_t)stream, dsq_all, dsq_len, chunks, nchunk, f1, cmw, wins, -1, nullptr);
     if (rc) return rc;
     *n_out = (int32_t)wins.size();
     if ((int64_t)wins.size() > cap) {

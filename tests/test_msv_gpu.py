@@ -144,3 +144,22 @@ def test_ssv_rejects_bad_residues_and_windows():
         f.f1_windows_batch(fr, np.array([(0, 1, 1000)], N.WINDOW_DTYPE), 0.1, 60)
     with pytest.raises(N.CmgpuError):
         f.f1_windows_batch(fr, np.array([(0, 1, 5000)], N.WINDOW_DTYPE), 0.1, 60)
+
+
+@pytest.mark.parametrize("m,f1,l", [(100, 0.9, 70001), (128, 0.5, 70001), (130, 0.02, 66000), (33, 0.35, 255)])
+def test_ssv_runs_across_segments(m, f1, l):
+    """Runs of triggers that cross segment borders, more than 256 segments to a chunk (256 residues each at
+    these lengths), candidates exactly 2M rows apart, and segments without any."""
+    p, cons = peaked_profile(70 + m, m)
+    seqs = [planted_frame(200, l, cons, 40), planted_frame(201, 300, cons, 1), planted_frame(202, l // 3, cons, 0)]
+    a = seqs[0]
+    for q, at in enumerate(range(2000, min(l - 4 * m, 40000), 2 * m)):  # plants one period of 2M rows apart
+        if q % 3 < 2:
+            a[at:at + m] = cons[:m]
+    buf, wins, offs, lens = frames_of(seqs)
+    _, _, oraw, orsc = oracle.f1_msv_windows(m, p.mat, p.trans, int(1.25 * m), -8.0, 0.69, buf, offs, lens, f1, m)
+    f = MsvFilter(p, int(1.25 * m), -8.0, 0.69)
+    raw = f.ssv_diagonals_batch(buf, wins, f1)
+    assert np.array_equal(np.stack([raw["chunk"], raw["n"], raw["length"], raw["k"]], 1), oraw) and len(oraw) > 0
+    assert same_f32(raw["score"], orsc)
+    f.close()
