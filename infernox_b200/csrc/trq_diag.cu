@@ -26,7 +26,7 @@
 // Cells of spans beyond a column's own start hold values nobody reads.
 //
 // Measured on one B200, 200 cut sequences of about 107 nt, non-banded Inside,
-// M = 379: 175 ms with the column wavefront of trq_scan.cu, 37 ms here.
+// M = 379: 175 ms with the column wavefront of trq_scan.cu, 23 ms here.
 // Bound: the latency of one warp's log-sum chains (one to two windows per
 // SM, four warps each); DRAM 2%.
 #include <climits>
@@ -141,9 +141,12 @@ __device__ __forceinline__ void node(const Params &p, Ctx &c, const Node *np, in
     int ihi = min(rhi, min(p.dx0, min(chi, p.W1 - 1) - 2));
 #pragma unroll
     for (int q = 0; q < NSPLIT + NI; q++) ihi = min(ihi, (int)np->dx[q]);
-    if (cend || skip || ((endmask | beginmask) & ~1)) ihi = -1;
+    constexpr int INS = (HAS_IL ? 1 << QIL : 0) | (HAS_IR ? 1 << QIR : 0);
+    if (cend || skip || (endmask & ~1) || (beginmask & ~(1 | INS))) ihi = -1;
     const bool end0 = (endmask & 1) != 0, beg0 = (beginmask & 1) != 0;
-    const T es0 = end0 ? S::ldg(p.endsc + v0) : Z, pen0 = beg0 ? S::ldg(p.pty + v0) : Z;
+    const bool begil = HAS_IL && (beginmask >> QIL & 1), begir = HAS_IR && (beginmask >> QIR & 1);
+    const T es0 = end0 ? S::ldg(p.endsc + v0) : Z, pen0 = beg0 ? S::ldg(p.pty + v0) : Z,
+            penil = begil ? S::ldg(p.pty + v0 + QIL) : Z, penir = begir ? S::ldg(p.pty + v0 + QIR) : Z;
 
     T ts[NSPLIT][CN], til[HAS_IL ? CN : 1], tir[HAS_IR ? NN + 1 : 1];
 #pragma unroll
@@ -214,8 +217,10 @@ __device__ __forceinline__ void node(const Params &p, Ctx &c, const Node *np, in
         }
         // One span; px, po: rows d of the child (column j) and of the outputs.
         // The inner version needs no test: every state in band, d >= 2, the
-        // child rows stored, at most the first state with a local end or a
-        // begin.  Planes L and R are computed in every pass; J does not read
+        // child rows stored, at most the first state with a local end, begins
+        // in it and the inserts only (where cm_tr_penalties puts them: without
+        // the inserts no node with begins took it, and the scan below 35 ms).
+        // Planes L and R are computed in every pass; J does not read
         // them, and a pass without one posts no begin from it.
         auto step = [&](auto inner_c, const uint32_t *px, uint32_t *o) {
             constexpr bool INNER = decltype(inner_c)::value;
@@ -232,7 +237,7 @@ __device__ __forceinline__ void node(const Params &p, Ctx &c, const Node *np, in
                 }
             }
             // the ROOT row's best begins so far
-            const bool post0 = INNER ? beg0 : beginmask && d >= 1 && d <= p.dx0;
+            const bool post0 = INNER ? beginmask != 0 : beginmask && d >= 1 && d <= p.dx0;
             uint32_t *rb = c.rbm + (int64_t)d * COLS + c.col, *ry = c.rby + (int64_t)d * COLS + c.col;
             T b0 = Z, b1 = Z, b2 = Z;
             if (post0) {
@@ -262,12 +267,13 @@ __device__ __forceinline__ void node(const Params &p, Ctx &c, const Node *np, in
             int yj = INT_MAX, yl = INT_MAX, yr = INT_MAX;
             auto begin = [&](int q, T J, T L, T R) {
                 if (INNER) {
-                    if (q == 0) {
-                        mj = S::add(J, pen0);
-                        ml = S::add(L, pen0);
-                        mr = S::add(R, pen0);
-                        yj = yl = yr = v0;
-                    }
+                    if (q != 0 && q != QIL && q != QIR) return;
+                    if (q == 0 ? !beg0 : q == QIL && HAS_IL ? !begil : !begir) return;
+                    const T pen = q == 0 ? pen0 : q == QIL && HAS_IL ? penil : penir;
+                    const T xj = S::add(J, pen), xl = S::add(L, pen), xr = S::add(R, pen);
+                    if (xj >= mj) mj = xj, yj = v0 + q;
+                    if (xl >= ml) ml = xl, yl = v0 + q;
+                    if (xr >= mr) mr = xr, yr = v0 + q;
                     return;
                 }
                 if (!(beginmask >> q & 1)) return;
