@@ -325,12 +325,15 @@ __global__ void __launch_bounds__(256) fwd_kernel(const float *__restrict__ tab,
 // registers: NQ = nq exactly (one instantiation per segment length, so no
 // cell needs a bounds test), the lane's seven transition values of a cell
 // read from shared memory as two 16-byte words, D->D read per pass.  LAZY:
-// M >= 100, the D passes stop at the first one that changes no cell.
-template <int NQ, bool LAZY>
-__global__ void __launch_bounds__(128, 3) fwd_kernel_reg(const float *__restrict__ ptab, int rq,
-                                                      const uint8_t *__restrict__ dsq,
-                                                      const FwdWin *__restrict__ wins, int nwin,
-                                                      int *__restrict__ next, float2 *__restrict__ out) {
+// M >= 100, the D passes stop at the first one that changes no cell.  A warp
+// works on `groups` windows at a time, eight at most.  Bound: the latency of a
+// warp's row with few windows, issue with many; the two together, M = 120,
+// 13,334 windows of 300: 0.75 ms, 640 Gcells/s.
+template <int NQ, bool LAZY, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) fwd_kernel_reg(const float *__restrict__ ptab, int rq,
+                                                            const uint8_t *__restrict__ dsq,
+                                                            const FwdWin *__restrict__ wins, int nwin, int groups,
+                                                            int *__restrict__ next, float2 *__restrict__ out) {
     extern __shared__ __align__(16) float sm[];
     const int tabn = NQ * T_N * 4 + KP * rq * 4;
     for (int q = threadIdx.x; q < tabn; q += blockDim.x) sm[q] = ptab[q];
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(128, 3) fwd_kernel_reg(const float *__restrict
     const float4 *T4 = reinterpret_cast<const float4 *>(sm) + z * 2;
     const float *TD = sm + z * T_N + T_DD;
     const float *R0 = sm + NQ * T_N * 4 + z;
+    if (lane >= groups * 4) return;  // this warp works on fewer windows
     float mmv[NQ], dmv[NQ], imv[NQ];
     for (;;) {
         int w = 0;
@@ -429,14 +433,24 @@ __global__ void __launch_bounds__(128, 3) fwd_kernel_reg(const float *__restrict
     }
 }
 
-typedef void (*FwdRegFn)(const float *, int, const uint8_t *, const FwdWin *, int, int *, float2 *);
+typedef void (*FwdRegFn)(const float *, int, const uint8_t *, const FwdWin *, int, int, int *, float2 *);
+
+// From this segment length on the 168 registers of three CTAs per SM hold the
+// kernel back (from 29 on it spills parts of the rows): there is a second build
+// for two CTAs (M = 98, one window: 0.162 -> 0.152 ms, M = 128 0.431 -> 0.350).  Shorter
+// segments were not tried: their rows take less than half of the 168.
+constexpr int FWD_WIDE_NQ = 25;
 
 // the register kernel for segment length nq (2..32) and the D-pass rule
-template <int... Q>
-FwdRegFn fwd_reg_kernel(int nq, bool lazy, std::integer_sequence<int, Q...>) {
-    static const FwdRegFn fixed[] = {fwd_kernel_reg<Q + 2, false>...};
-    static const FwdRegFn early[] = {fwd_kernel_reg<Q + 2, true>...};
-    return (lazy ? early : fixed)[nq - 2];
+template <int CTAS, int FROM, int... Q>
+FwdRegFn fwd_reg_pick(int nq, bool lazy, std::integer_sequence<int, Q...>) {
+    static const FwdRegFn fixed[] = {fwd_kernel_reg<Q + FROM, false, CTAS>...};
+    static const FwdRegFn early[] = {fwd_kernel_reg<Q + FROM, true, CTAS>...};
+    return (lazy ? early : fixed)[nq - FROM];
+}
+FwdRegFn fwd_reg_kernel(int nq, bool lazy, bool wide) {
+    return wide ? fwd_reg_pick<2, FWD_WIDE_NQ>(nq, lazy, std::make_integer_sequence<int, 33 - FWD_WIDE_NQ>())
+                : fwd_reg_pick<3, 2>(nq, lazy, std::make_integer_sequence<int, 31>());
 }
 
 // bias_filter_score before its length term, one thread per window
@@ -594,13 +608,25 @@ int score_windows(const cmgpu_fwd_filter *f, cudaStream_t st, const uint8_t *dsq
     const bool regs = nq <= 32 && f->kernel != CMGPU_FWD_KERNEL_SHARED;
     if (nf > 0 && regs) {
         // the segment of each lane fits in registers
-        auto kern = cmx::dev::fwd_reg_kernel(nq, h.M >= 100, std::make_integer_sequence<int, 31>());
+        // A batch that two CTAs per SM hold takes the build for two where that one
+        // exists (M = 120: one window 0.373 -> 0.316 ms, 6,000 windows of 300 0.568 ->
+        // 0.535; 13,334 windows, which fill three CTAs, 0.750 against 1.02).
+        const bool wide = nq >= cmx::dev::FWD_WIDE_NQ && nf <= (int64_t)sms * 2 * 32;
+        auto kern = cmx::dev::fwd_reg_kernel(nq, h.M >= 100, wide);
         const size_t rsmem = (size_t)(nq * T_N * 4 + KP * h.rq * 4) * sizeof(float);
         FWD_TRY(cmx::allow_max_dynamic_smem(kern));
         int per_sm = 0;
         FWD_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, rsmem));
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((nf + 31) / 32, (int64_t)sms * std::max(per_sm, 1)));
-        kern<<<grid, 128, rsmem, st>>>(f->d_ptab, h.rq, d_dsq, d_w, nf, d_next, d_out);
+        // Windows per warp: first one warp per scheduler (four per SM), then
+        // more windows in each.  The groups of a warp part ways in the D
+        // passes, so few windows spread out (500 of 300: 0.445 -> 0.385 ms,
+        // 0.332 with the build for two; 3,000: 0.455 -> 0.375); more warps with few windows each are
+        // slower, as the unrolled row does not stay in the instruction cache (3,000 on
+        // eight warps per SM: 0.70 ms against 0.455).
+        const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(8, (nf + sms * 4 - 1) / (sms * 4)));
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((nf + 4 * groups - 1) / (4 * groups),
+                                                                    (int64_t)sms * std::max(per_sm, 1)));
+        kern<<<grid, 128, rsmem, st>>>(f->d_ptab, h.rq, d_dsq, d_w, nf, groups, d_next, d_out);
         FWD_TRY(cudaGetLastError());
         mf->last_launches++;
     } else if (nf > 0) {

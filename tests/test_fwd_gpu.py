@@ -83,6 +83,24 @@ def test_fwd_long_windows_planted_homologs(m, shared):
     f.close()
 
 
+@pytest.mark.parametrize("m", [60, 96, 97, 100, 113, 128])
+@pytest.mark.parametrize("nwin", [3, 593, 4737, 10001])
+def test_fwd_batch_sizes(m, nwin):
+    """Batches around the switches of the windows per warp and of the build
+    with more registers (segment lengths from 25 on), uneven and empty windows."""
+    p, cons = peaked_profile(3 + m, m, peak=0.7)
+    f = FwdFilter(p, mean_composition(p))
+    buf = planted_frame(5 + m, 4000, cons, 9)
+    r = np.random.default_rng(nwin)
+    wins = np.zeros(nwin, N.WINDOW_DTYPE)
+    wins["i0"] = r.integers(1, 3900, nwin)
+    wins["j0"] = wins["i0"] - 1 + r.integers(0, 90, nwin)
+    fs, _ = f.score_batch(buf, wins, bias=False)
+    ofs, _, _ = oracle.fwd_score_batch(m, p.mat, p.trans, buf, list(wins["i0"] - 1), list(wins["j0"] - wins["i0"] + 1))
+    assert np.array_equal(bits(fs), bits(ofs))
+    f.close()
+
+
 def test_fwd_windows_inside_frames_in_any_order():
     """Windows cut from one frame at any offsets, uneven lengths, one empty."""
     rng = Lcg(77)
