@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -26,7 +27,12 @@ void on_cores(size_t n, size_t work, size_t grain, F f) {
         for (size_t k; (k = next.fetch_add(1)) < n;) f(k);
     };
     std::vector<std::thread> pool;
-    for (size_t t = 1; t < nthr; t++) pool.emplace_back(run);
+    pool.reserve(nthr);
+    try {
+        for (size_t t = 1; t < nthr; t++) pool.emplace_back(run);
+    } catch (const std::system_error &) {
+        // no more threads to be had: those there are, and this one, do the work
+    }
     run();
     for (auto &th : pool) th.join();
 }
