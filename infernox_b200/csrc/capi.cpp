@@ -652,7 +652,13 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     // well inside it, so the scan is not repeated with a larger buffer.
     // cmcalibrate's scan has no cutoff: in a glocal model a dozen cells of a
     // column exceed all shorter ones.
-    const size_t per_cand = calib ? (size_t)total_cols * 18 : (size_t)(total_cols / 4);
+    size_t per_cand = (size_t)(total_cols / 4);
+    if (calib) {
+        // ... within a quarter of the free memory: a scan that needs more is repeated
+        size_t freeb = 0, totalb = 0;
+        CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+        per_cand = std::max(per_cand, std::min((size_t)total_cols * 18, freeb / 4 / sizeof(Cand)));
+    }
     const size_t cand_cap = std::max<size_t>({ws->cands_cap, (size_t)1 << 16, per_cand});
     if ((rc = ensure_dev(&ws->d_cands, &ws->cands_cap, cand_cap))) return rc;
     if (!diag && !sweep && !deck_smem && (int64_t)items.size() < best_l) {
