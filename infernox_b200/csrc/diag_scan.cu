@@ -41,7 +41,7 @@
 //
 // Measured on one B200 (before: the level kernel of qdb_scan.cu): Inside,
 // non-banded, M = 379, W = 148, 296 windows of 512: 220 Gcells/s, CYK 335; two
-// 1 kb windows of a 4,629-state model, CYK: 1,809 -> 50 ms.  Bound: the
+// 1 kb windows of a 4,629-state model, CYK: 1,809 -> 53 ms.  Bound: the
 // latency of the log-sum chains (LDS and dependent ALU) at 16 warps per SM,
 // 53% of issue slots; DRAM 21%.
 #include <cuda_runtime.h>

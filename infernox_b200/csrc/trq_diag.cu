@@ -10,7 +10,7 @@
 // residue and read span d of states below), so a node computes IR first, then
 // IL, then its split states.  Inserts stay in registers; of the next node
 // only the split states' planes are loaded, two spans ahead.  Warps run
-// skewed by one 16-span phase with one CTA barrier per phase, as there.
+// skewed by one 16-span phase with one CTA barrier per phase.
 //
 // ROOT.  The reference never resets its ROOT row: a truncated begin counts
 // only if it exceeds the best one of every earlier column of the same parity
