@@ -799,6 +799,12 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             if (rows > 0) c.gsteps += (rows + DG_CHUNK - 1) / DG_CHUNK;
         }
         for (int g0 = 0; g0 < c.ncols; g0 += cols) {
+            // The right neighbour has finished the whole group before: the node
+            // buffers start again with the first one, which in a third of the
+            // models is the one ROOT still reads its child from (and a group of
+            // fewer steps than the slack would let a warp run two ahead).  About
+            // a step of waiting per group of a thousand.
+            if (c.w < c.nw - 1) dg_wait(c, c.w + 1, c.step);
             c.first = g0 == 0;
             c.last = g0 + cols >= c.ncols;
             c.jrel = g0 + c.col;

@@ -69,3 +69,21 @@ def test_calibration_scan_matches_level_kernel(sr, null3):
         x = a.calibrate_scan_batch(sr, QDB2, buf, w, null3)
         y = b.calibrate_scan_batch(sr, QDB2, buf, w, null3)
         assert len(x) > 0 and x.tobytes() == y.tobytes()
+
+
+# (chunk: residues reported per item, which adds W-1 columns before them; a
+# group of columns holds 512 at most, so 1,152 takes three groups and 500 two.
+# small2 has 44 nodes that own a buffer, two more than a multiple of three, and
+# a ROOT of five steps of sixteen spans.)
+@pytest.mark.parametrize("chunk,n", [(500, 1400), (1152, 3000)])
+@pytest.mark.parametrize("name", ["small0", "trna", "small2", "mb3"])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, QDB2), (INSIDE_I32, NOQDB)])
+def test_glocal_column_groups_match_level_kernel(name, sr, band, chunk, n):
+    cm, g, _ = models(name)
+    a, b = scan.Scanner(g), scan.Scanner(g)
+    b.set_kernel(KERNEL_LEVEL)
+    a.set_shape(0, 0, chunk, 0)
+    dsq = frame(seq_of(cm, n, n))
+    ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
+    assert a.stats()["kernel"] == DIAG and len(ca) > n
+    assert ca == cb
