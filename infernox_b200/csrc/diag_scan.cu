@@ -820,6 +820,7 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             if (p.local && c.jmax > 0)
                 for (int d = p.root_dn; d <= min(p.root_dxcap, c.jmax); d++)
                     S::st(c.reg + c.col + (int64_t)d * DG_COLS, NONE);
+            __syncwarp();  // the first node's fetch copies the begin row of every lane
             for (int n = 0; n < p.nnodes; n++) {
                 const DgNode *np = p.nodes + n;
                 dg_begin_node(c);

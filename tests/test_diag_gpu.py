@@ -87,3 +87,19 @@ def test_glocal_column_groups_match_level_kernel(name, sr, band, chunk, n):
     ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
     assert a.stats()["kernel"] == DIAG and len(ca) > n
     assert ca == cb
+
+
+# Local begins start from an empty row in every group of columns: the row of
+# the group before it must be gone when the first node reads it.
+@pytest.mark.parametrize("chunk,n", [(500, 1400), (1152, 3000)])
+@pytest.mark.parametrize("name", ["small0", "small2", "mb3"])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, NOQDB)])
+def test_local_begins_of_column_groups_match_level_kernel(name, sr, band, chunk, n):
+    cm, _, l = models(name)
+    a, b = scan.Scanner(l), scan.Scanner(l)
+    b.set_kernel(KERNEL_LEVEL)
+    a.set_shape(0, 0, chunk, 0)
+    dsq = frame(seq_of(cm, n, 7 * n))
+    ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
+    assert a.stats()["kernel"] == DIAG and len(ca) > n
+    assert ca == cb
