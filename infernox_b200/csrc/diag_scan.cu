@@ -362,12 +362,15 @@ __device__ __forceinline__ void dg_node(const DgParams &p, DgCtx &c, const DgNod
             xl1[y] = ldx(y, d - 1, 1);
         }
     }
-    int ci = HAS_IL ? c.ring[(c.jrel - d + 1) & c.rmask] : 0;  // residue j-d+1
+    int ci = 0;  // residue j-d+1
     for (int r0 = rlo; r0 <= rhi; r0 += DG_CHUNK) {
         const int rend = min(r0 + DG_CHUNK - 1, rhi);
         const int dstop = min(rend, c.jmax);
         const int slot = c.step & (DG_XCH - 1);
         dg_begin_step(c);
+        // after the wait: before a group's first step the warps on the left may
+        // not have written their residues
+        if (HAS_IL) ci = c.ring[(c.jrel - r0 + 1) & c.rmask];
         // the inserts of the column left of the warp: lane r holds span r0 + r
         T hil = ZERO, hir = ZERO;
         if constexpr (HAS_IR) {

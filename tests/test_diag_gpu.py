@@ -3,6 +3,8 @@ tiling can go wrong: a warp's 32 columns, a CTA's group of columns, the last
 partial group, windows shorter than W, forced pieces -- against the oracle
 bit for bit, and every ROOT cell against the level kernel over all semirings,
 band sets and configurations."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -103,3 +105,23 @@ def test_local_begins_of_column_groups_match_level_kernel(name, sr, band, chunk,
     ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
     assert a.stats()["kernel"] == DIAG and len(ca) > n
     assert ca == cb
+
+
+# Bands that begin at span 5 in every state: the first node of a group then
+# starts with residues of the warps on its left.
+@pytest.mark.parametrize("name", ["small0", "mb3"])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, QDB2)])
+def test_bands_without_short_spans_match_oracle(name, sr, band):
+    cm, _, _ = models(name)
+    ref = oracle_cfg(name, True)
+    up = {k: np.where(np.asarray(ref.sttype) == 7, getattr(ref, k), np.maximum(getattr(ref, k), 5)).astype(np.int32)
+          for k in ("dmin1", "dmin2")}
+    up.update({k: np.maximum(getattr(ref, k), up["dmin" + k[-1]]).astype(np.int32) for k in ("dmax1", "dmax2")})
+    c = dataclasses.replace(ref, **up)
+    s = scan.Scanner(c)
+    for n in (40, 700):
+        dsq = frame(seq_of(cm, n, 3 * n))
+        want, _, _, _ = oracle.qdb_scan(c, sr, band, dsq, 1, n, -60.0, True)
+        got = s.generic_scan(sr, band, dsq, 1, n, -60.0, True)
+        assert s.stats()["kernel"] == DIAG
+        assert len(want) > 0 and bits(got) == bits(want)
