@@ -704,7 +704,9 @@ __device__ __forceinline__ void dg_bif(const DgParams &p, DgCtx &c, const DgNode
                 S::st(o, x);
                 if (need_left) {
                     // the column left of the group, and the group's last one
+                    // (which takes its place: one warp may hold both)
                     if (c.w == 0 && c.lane == 0) S::st(o - 1, c.first ? fill : S::ld(bnd + (d - rlo) * DG_SLOTS));
+                    __syncwarp();
                     if (!c.last && c.w == c.nw - 1 && c.lane == 31) S::st(bnd + (d - rlo) * DG_SLOTS, x);
                 }
                 if (p.local && beg && in && d >= p.root_dn && d <= p.root_dxcap) {

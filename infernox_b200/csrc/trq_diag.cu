@@ -600,6 +600,7 @@ __device__ __forceinline__ void bif(const Params &p, Ctx &c, const Node *np, int
                         S::st(o - 1, c.first ? b0 : S::ld(b));
                         S::st(o + 2 * PITCH - 1, c.first ? Z : S::ld(b + 2));
                     }
+                    __syncwarp();  // (one warp may hold both columns)
                     if (!c.last && c.w == c.nw - 1 && c.lane == 31) {
                         S::st(b, J);
                         S::st(b + 2, R);
