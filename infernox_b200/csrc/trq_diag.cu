@@ -10,7 +10,10 @@
 // residue and read span d of states below), so a node computes IR first, then
 // IL, then its split states.  Inserts stay in registers; of the next node
 // only the split states' planes are loaded, two spans ahead.  Warps run
-// skewed by one 16-span phase with one CTA barrier per phase.
+// skewed by one 16-span phase with one CTA barrier per phase.  (So the last
+// warp has finished a phase of a group before the first one reaches the same
+// phase of the next group, if a group has at least as many phases as the CTA
+// warps; the launch takes fewer warps where it has not.)
 //
 // ROOT.  The reference never resets its ROOT row: a truncated begin counts
 // only if it exceeds the best one of every earlier column of the same parity
@@ -803,6 +806,12 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 1) kernel(const __grid_constan
         }
         __syncthreads();
     }
+}
+
+int64_t group_phases(const std::vector<Node> &nodes, int span) {
+    int64_t n = 1;  // ROOT's begins
+    for (const Node &x : nodes) n += (std::min((int)x.rhi, span) + CHUNK) / CHUNK;
+    return n;
 }
 
 static size_t smem_bytes(const Params &p, int warps) {

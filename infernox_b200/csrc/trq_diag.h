@@ -74,6 +74,8 @@ struct Params {
 // words of one CTA's region for windows spanning at most W1 - 1
 int64_t region_words(const Params &p);
 int occupancy(const Params &p, int warps);
+// phases a warp takes for one group of columns of a window spanning `span`
+int64_t group_phases(const std::vector<Node> &nodes, int span);
 cudaError_t launch(const Params &p, int ctas, int warps, cudaStream_t s);
 
 // The nodes of a model for band caps dxcap (false: another node topology, or

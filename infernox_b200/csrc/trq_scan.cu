@@ -977,6 +977,14 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
         // no more warps than the longest window has columns
         const int longest = wl[0].j0 - wl[0].i0 + 1;
         warps = std::min(trqd::MAX_WARPS, (longest + 31) / 32);
+        // a window of several groups of columns has as many phases per group
+        // as warps, or more (a model of a few nodes with a short W has not)
+        for (; warps > 1; warps--) {
+            int span = INT_MAX;
+            for (const trq::Win &x : wl)
+                if (x.j0 - x.i0 + 1 > 32 * warps) span = std::min(span, x.w);
+            if (span == INT_MAX || trqd::group_phases(nodes, span) >= warps) break;
+        }
         dgp.ring_cols = (dgp.W1 + trqd::COLS + 31) & ~31;
         dgp.ring_len = 1;
         while (dgp.ring_len < dgp.W1 + 64 * warps) dgp.ring_len <<= 1;

@@ -14,6 +14,7 @@ import torch
 
 import oracle
 from infernox_b200 import _native as N
+from infernox_b200 import model, synth
 from infernox_b200.hb import (TrInputs, hb_scan_batch, ref_itr_inside_scan, ref_tr_cyk_scan, tr_scan_hb_batch)
 from infernox_b200.scan import CYK_F32, INSIDE_I32, NOQDB, QDB1, QDB2, Scanner
 
@@ -109,3 +110,26 @@ def test_long_hit_lists_match_oracle(sr, band):
     got = Scanner(l).generic_scan(sr, band, dsq, 1, n, -60.0, True)
     assert [(h[0], h[1], bits(h[2]), bits(h[3])) for h in got] == [(h[0], h[1], bits(h[2]), bits(h[3])) for h in ref]
     assert len(ref) > 0
+
+
+# Models of three and five nodes with W of 5 and 10 to 12: a group of columns
+# takes fewer phases than eight warps, so the launch takes fewer.
+@pytest.mark.parametrize("ss", ["..", "....", "(...)"])
+@pytest.mark.parametrize("loc", [False, True])
+@pytest.mark.parametrize("qdb", [NOQDB, QDB2])
+def test_truncated_scan_of_tiny_models(ss, loc, qdb):
+    cm = synth.synth_cm(ss, 1, name="tiny", ins_open=0.005, ins_self=0.1)
+    cfg = model.configure(cm, local=loc)
+    assert cfg.W <= 15
+    sc = Scanner(cfg)
+    tt = tr_tables(cm, cfg, 4, loc)
+    for n in (200, 257, 700, 1100):
+        f = frame(planted_seq(cm, n, 0.5, 12, seed=n, degenerate=0.02))
+        for inside, fn in ((False, ref_tr_cyk_scan), (True, ref_itr_inside_scan)):
+            ro = oracle.trq_scan(cfg, inside, tt, f, 1, n, -6.0, True, qdb, 4, loc)
+            go = fn(sc, tri_of(tt, loc), f, 1, n, -6.0, qdb, True, 4)
+            assert len(ro[0]) > 0
+            assert bits(go[1]) == bits(ro[1]) and go[2] == ro[2] and bits(go[3]) == bits(ro[3])
+            assert [(a, b, bits(s), bits(e), m, r) for a, b, s, e, m, r in go[0]] == \
+                   [(a, b, bits(s), bits(e), m, r) for a, b, s, e, m, r in ro[0]]
+    sc.close()
