@@ -10,7 +10,7 @@ import pytest
 
 import oracle
 from infernox_b200 import _native as N
-from infernox_b200 import scan
+from infernox_b200 import model, scan, synth
 from infernox_b200.scan import CYK_F32, INSIDE_I32, KERNEL_LEVEL, NOQDB, QDB1, QDB2
 
 from helpers import frame, models, oracle_cfg, planted_seq
@@ -125,3 +125,21 @@ def test_bands_without_short_spans_match_oracle(name, sr, band):
         got = s.generic_scan(sr, band, dsq, 1, n, -60.0, True)
         assert s.stats()["kernel"] == DIAG
         assert len(want) > 0 and bits(got) == bits(want)
+
+
+# Models of three and five nodes: a group of columns takes fewer steps than a
+# warp may be ahead of its right neighbour.
+@pytest.mark.parametrize("ss", ["..", "....", "(...)"])
+@pytest.mark.parametrize("local", [False, True])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, QDB2), (INSIDE_I32, NOQDB)])
+def test_tiny_models_match_level_kernel(ss, local, sr, band):
+    cm = synth.synth_cm(ss, 1, name="tiny", ins_open=0.005, ins_self=0.1)
+    c = model.configure(cm, local=local)
+    a, b = scan.Scanner(c), scan.Scanner(c)
+    b.set_kernel(KERNEL_LEVEL)
+    for n, chunk in ((257, 0), (3000, 0), (3000, 1152)):
+        a.set_shape(0, 0, chunk, 0)
+        dsq = frame(seq_of(cm, n, n))
+        ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
+        assert (a.stats()["kernel"], b.stats()["kernel"]) == (DIAG, KERNEL_LEVEL)
+        assert len(ca) > n and ca == cb
