@@ -6,6 +6,8 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <iterator>
+#include <map>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -61,11 +63,15 @@ void replay_cells(const C *c, size_t n, size_t nwin, std::vector<C> &out, F repo
 
 // remove_overlaps_greedy (src/cp9.rs:6544-6574, src/cm_dpsearch_trunc.rs:2470):
 // hits by score (descending, stable) then start; a hit is removed when it
-// overlaps an earlier hit that was kept.  Most hits overlap one of the best
-// ones, so only the best part is sorted, and what overlaps the hits kept so far
-// is dropped before the next part is: the same hits in the same order, without
-// sorting them all (150,000 hits of one window: 19 ms sorted).  The kept hits
-// are disjoint, so a count of covered residues tells an overlap.
+// overlaps an earlier hit that was kept.  The kept hits are disjoint.
+//
+// Lists with a hit per 32 residues or more (150,000 hits of one window: 19 ms
+// when they were all sorted): most hits overlap one of the best ones, so only
+// the best part is sorted, and what overlaps the hits kept so far is dropped
+// before the next part is; a count of covered residues tells an overlap.  That
+// takes five bytes per residue between the first and the last hit, so lists
+// with fewer hits are sorted whole, and the kept hit with the largest start
+// <= j is looked up in a map: memory follows the hits in both.
 template <class H>
 void remove_overlaps(std::vector<H> &h) {
     if (h.size() < 2) return;
@@ -73,6 +79,21 @@ void remove_overlaps(std::vector<H> &h) {
     for (const H &x : h) {
         lo = std::min(lo, std::min(x.i, x.j));
         hi = std::max(hi, std::max(x.i, x.j));
+    }
+    if ((size_t)(hi - lo) / 32 > h.size()) {
+        std::stable_sort(h.begin(), h.end(), [](const H &a, const H &b) {
+            return a.score != b.score ? a.score > b.score : a.i < b.i;
+        });
+        std::map<decltype(lo), decltype(lo)> kept;  // start -> end
+        size_t o = 0;
+        for (size_t k = 0; k < h.size(); k++) {
+            const auto it = kept.upper_bound(h[k].j);
+            if (it != kept.begin() && std::prev(it)->second >= h[k].i) continue;
+            kept.emplace(h[k].i, h[k].j);
+            h[o++] = h[k];
+        }
+        h.resize(o);
+        return;
     }
     std::vector<char> mark((size_t)(hi - lo + 1), 0);
     std::vector<int32_t> upto((size_t)(hi - lo + 2), 0);  // covered residues before lo + x
