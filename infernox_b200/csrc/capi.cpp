@@ -322,10 +322,10 @@ struct WinDesc {
     int32_t i0, j0;
 };
 
-static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbidx, const uint8_t *d_dsq,
-                    const uint8_t *h_dsq, int64_t dsq_len, const std::vector<WinDesc> &wins, float cutoff,
-                    int do_null3, bool plain, std::vector<std::vector<cmgpu_hit>> &hits_per_win,
-                    std::vector<Cand> *cells_out = nullptr, bool calib = false) {
+static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbidx, const uint8_t *d_dsq,
+                        const uint8_t *h_dsq, int64_t dsq_len, const std::vector<WinDesc> &wins, float cutoff,
+                        int do_null3, bool plain, std::vector<std::vector<cmgpu_hit>> &hits_per_win,
+                        std::vector<Cand> *cells_out, bool calib) {
     if (semiring != CMGPU_CYK_F32 && semiring != CMGPU_INSIDE_I32) {
         set_error("unknown semiring");
         return CMGPU_EINVAL;
@@ -903,6 +903,16 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
     });
     (void)dsq_len;
     return CMGPU_OK;
+}
+
+static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbidx, const uint8_t *d_dsq,
+                    const uint8_t *h_dsq, int64_t dsq_len, const std::vector<WinDesc> &wins, float cutoff,
+                    int do_null3, bool plain, std::vector<std::vector<cmgpu_hit>> &hits_per_win,
+                    std::vector<Cand> *cells_out = nullptr, bool calib = false) {
+    return host_memory_checked([&]() {
+        return scan_windows(m, ws, semiring, qdbidx, d_dsq, h_dsq, dsq_len, wins, cutoff, do_null3, plain,
+                            hits_per_win, cells_out, calib);
+    });
 }
 
 static bool check_codes(const uint8_t *dsq, int32_t n);

@@ -1520,8 +1520,10 @@ int hb_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int report, i
     while (e0 < ntask) {
         int32_t e1 = e0 + 1;
         while (e1 < ntask && alpha_off[e1 + 1] - alpha_off[e0] <= budget) e1++;
-        rc = hb_launch(m, h, st, semiring, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin, row_pin,
-                       row_base, alpha_off, results, hits, ms, launches);
+        rc = host_memory_checked([&]() {
+            return hb_launch(m, h, st, semiring, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin, row_pin,
+                             row_base, alpha_off, results, hits, ms, launches);
+        });
         if (rc) return rc;
         e0 = e1;
     }
@@ -1743,8 +1745,10 @@ int tr_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, const cmgpu_t
     while (e0 < ntask) {
         int32_t e1 = e0 + 1;
         while (e1 < ntask && alpha_off[e1 + 1] - alpha_off[e0] <= budget) e1++;
-        rc = tr_launch(m, h, st, semiring, trt, cx, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin,
-                       row_pin, row_base, alpha_off, results, hits, ms, launches);
+        rc = host_memory_checked([&]() {
+            return tr_launch(m, h, st, semiring, trt, cx, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin,
+                             row_pin, row_base, alpha_off, results, hits, ms, launches);
+        });
         if (rc) return rc;
         e0 = e1;
     }

@@ -7,6 +7,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -20,6 +21,20 @@
 namespace cmx {
 
 void set_error(const std::string &msg);
+
+// A scan's status, host memory that cannot be had included: what a scan
+// allocates per cell or window grows with the call, and no exception leaves
+// the C entry points.
+template <class F>
+int host_memory_checked(F scan) {
+    try {
+        return scan();
+    } catch (const std::bad_alloc &) {
+        set_error("host allocation failed");
+        return CMGPU_ENOMEM;
+    }
+}
+
 struct HbDev;  // device tables of the HMM-banded scanner (hb_scan.cu)
 void hb_free(HbDev *h);
 struct TrqDev;  // device tables of the truncated QDB / non-banded scanner (trq_scan.cu)

@@ -6,16 +6,18 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
 #include <iterator>
 #include <map>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 namespace cmx {
 
 // Runs f(0) .. f(n - 1) on up to one thread per `grain` units of work, at
-// most the host's cores; the items are taken in order.
+// most the host's cores; the items are taken in order.  What an item throws
+// reaches the caller once every thread has stopped (the first one thrown; the
+// items not begun by then are left out).
 template <class F>
 void on_cores(size_t n, size_t work, size_t grain, F f) {
     const size_t nthr = std::min<size_t>({n, (size_t)std::max(1u, std::thread::hardware_concurrency()),
@@ -25,18 +27,26 @@ void on_cores(size_t n, size_t work, size_t grain, F f) {
         return;
     }
     std::atomic<size_t> next{0};
+    std::atomic<bool> failed{false};
+    std::exception_ptr thrown;
     auto run = [&]() {
-        for (size_t k; (k = next.fetch_add(1)) < n;) f(k);
+        try {
+            for (size_t k; (k = next.fetch_add(1)) < n;) f(k);
+        } catch (...) {
+            next.store(n);
+            if (!failed.exchange(true)) thrown = std::current_exception();
+        }
     };
     std::vector<std::thread> pool;
     pool.reserve(nthr);
     try {
         for (size_t t = 1; t < nthr; t++) pool.emplace_back(run);
-    } catch (const std::system_error &) {
+    } catch (const std::exception &) {
         // no more threads to be had: those there are, and this one, do the work
     }
     run();
     for (auto &th : pool) th.join();
+    if (thrown) std::rethrow_exception(thrown);
 }
 
 // Cells c[0..n) of windows 0..nwin-1 (field env) -> `out` ordered by (window,

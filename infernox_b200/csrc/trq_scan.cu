@@ -1201,8 +1201,10 @@ extern "C" int cmgpu_tr_qdb_scan_batch(const cmgpu_model *m, void *stream, int s
     *n_out = 0;
     if (nwin == 0) return CMGPU_OK;
     std::vector<cmgpu_tr_hit> all;
-    int rc = trq_batch(m, (cudaStream_t)stream, semiring, qdbidx, tt, pass_idx, do_null3, dsq_all, dsq_len, wins,
-                       nwin, cutoff, results, all);
+    int rc = host_memory_checked([&]() {
+        return trq_batch(m, (cudaStream_t)stream, semiring, qdbidx, tt, pass_idx, do_null3, dsq_all, dsq_len, wins,
+                         nwin, cutoff, results, all);
+    });
     if (rc) return rc;
     *n_out = (int64_t)all.size();
     if ((int64_t)all.size() > cap) {
@@ -1226,8 +1228,10 @@ extern "C" int cmgpu_tr_qdb_scan(const cmgpu_model *m, int semiring, int qdbidx,
     const cmgpu_window wd{0, i0, j0};
     cmgpu_trq_result r{};
     std::vector<cmgpu_tr_hit> all;
-    int rc = trq_batch(m, nullptr, semiring, qdbidx, tt, pass_idx, do_null3, dsq, (int64_t)n + 2, &wd, 1, cutoff, &r,
-                       all);
+    int rc = host_memory_checked([&]() {
+        return trq_batch(m, nullptr, semiring, qdbidx, tt, pass_idx, do_null3, dsq, (int64_t)n + 2, &wd, 1, cutoff, &r,
+                         all);
+    });
     if (rc) return rc;
     *vsc_root = r.vsc_root;
     *vmode = r.vmode;

@@ -87,3 +87,31 @@ def run(tmp_path, name, source):
 def test_overlap_rule_and_its_memory(tmp_path):
     r = run(tmp_path, "overlaps", OVERLAPS)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+THROWS = PRELUDE + r"""
+int main() {
+    for (int bad : {0, 57, 199}) {
+        std::atomic<int> ran{0};
+        bool caught = false;
+        try {
+            cmx::on_cores(200, 200, 1, [&](size_t k) {
+                ran++;
+                if ((int)k == bad) throw std::bad_alloc();
+            });
+        } catch (const std::bad_alloc &) {
+            caught = true;
+        }
+        assert(caught && ran > bad);
+    }
+    std::atomic<int> ran{0};
+    cmx::on_cores(1000, 1000, 1, [&](size_t) { ran++; });
+    assert(ran == 1000);
+    return 0;
+}
+"""
+
+
+def test_what_an_item_throws_reaches_the_caller(tmp_path):
+    r = run(tmp_path, "throws", THROWS)
+    assert r.returncode == 0, r.stdout + r.stderr
