@@ -27,6 +27,7 @@
 #include "../../include/cmscan_gpu.h"
 #include "cm_internal.h"
 #include "model_internal.h"
+#include "plan_util.h"
 #include "qdb_kernel.h"
 #include "qdb_plan.h"
 #include "replay.h"
@@ -201,6 +202,27 @@ static int ensure_dev(T **p, size_t *cap, size_t n) {
     return CMGPU_OK;
 }
 
+// Room for `most` units of `unit` elements, or for as many as can be had down to
+// `least`; *got says how many (0: not even those).
+template <class T>
+static int ensure_units(T **p, size_t *cap, size_t unit, size_t most, size_t least, size_t *got) {
+    *got = most;
+    if (unit * most <= *cap && *p) return CMGPU_OK;
+    cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    cudaError_t e = cudaSuccess;
+    *got = most_that_fit(most, least, [&](size_t n) {
+        if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return false;
+        e = cudaMalloc((void **)p, unit * n * sizeof(T));
+        if (e == cudaSuccess) *cap = unit * n;
+        else cudaGetLastError();
+        return e == cudaSuccess;
+    });
+    if (*got == 0 && e != cudaErrorMemoryAllocation) CUDA_TRY(e);
+    return CMGPU_OK;
+}
+
 static int ensure_host_cands(cmgpu_workspace *ws, size_t n) {
     if (n <= ws->h_cands_cap && ws->h_cands) return CMGPU_OK;
     size_t nc = std::max<size_t>(n, ws->h_cands_cap * 3 / 2 + 16);
@@ -317,6 +339,10 @@ void report_window(const cmgpu_model *m, int semiring, const Cand *c, size_t n, 
 // ---------------------------------------------------------------------------
 constexpr int DIAG_WARPS = 8;  // warps per CTA of the diagonal kernel on full batches
 
+// scan_windows: no memory for one CTA of the diagonal kernel (its region holds
+// W rows and more per bifurcation; the level kernel's decks are smaller)
+constexpr int NO_DIAG_REGION = 1;
+
 struct WinDesc {
     int64_t off;
     int32_t i0, j0;
@@ -325,7 +351,7 @@ struct WinDesc {
 static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbidx, const uint8_t *d_dsq,
                         const uint8_t *h_dsq, int64_t dsq_len, const std::vector<WinDesc> &wins, float cutoff,
                         int do_null3, bool plain, std::vector<std::vector<cmgpu_hit>> &hits_per_win,
-                        std::vector<Cand> *cells_out, bool calib) {
+                        std::vector<Cand> *cells_out, bool calib, bool level) {
     if (semiring != CMGPU_CYK_F32 && semiring != CMGPU_INSIDE_I32) {
         set_error("unknown semiring");
         return CMGPU_EINVAL;
@@ -411,7 +437,7 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
     // cm_from_guide's node layout): faster at every size measured, 2.6 against
     // 26.8 ms for one 300-column window, 112 against 770 ms for 120 uneven
     // windows.  The level kernel takes the other models.
-    const bool diag = dp->dg_ok && ws->kernel == CMGPU_KERNEL_AUTO;
+    const bool diag = dp->dg_ok && ws->kernel == CMGPU_KERNEL_AUTO && !level;
     const bool sweep = dp->sw_ok && ws->kernel == CMGPU_KERNEL_SWEEP;
     const size_t SMEM_CAP = 227 * 1024 - 1024, SM_CAP = 228 * 1024;
     const int threads = ws->threads;
@@ -659,8 +685,15 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
         CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
         per_cand = std::max(per_cand, std::min((size_t)total_cols * 18, freeb / 4 / sizeof(Cand)));
     }
-    const size_t cand_cap = std::max<size_t>({ws->cands_cap, (size_t)1 << 16, per_cand});
-    if ((rc = ensure_dev(&ws->d_cands, &ws->cands_cap, cand_cap))) return rc;
+    const size_t cand_least = std::max<size_t>((size_t)1 << 16, (size_t)(total_cols / 4));
+    size_t cand_got = 0;
+    if ((rc = ensure_units(&ws->d_cands, &ws->cands_cap, 1, std::max({ws->cands_cap, cand_least, per_cand}),
+                           cand_least, &cand_got)))
+        return rc;
+    if (cand_got == 0) {
+        set_error("no device memory for the reportable cells");
+        return CMGPU_ENOMEM;
+    }
     if (!diag && !sweep && !deck_smem && (int64_t)items.size() < best_l) {
         // fewer work items than lanes: no deck for lanes that would stay idle
         best_l = (int)items.size();
@@ -691,7 +724,13 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
         const size_t have = freeb / 2 + ws->diag_cap * 4;
         ctas = (int)std::min<int64_t>((int64_t)items.size(), (int64_t)ws->sm_count * best_c);
         ctas = (int)std::min<size_t>((size_t)ctas, std::max<size_t>(1, have / std::max<size_t>(per_cta, 1)));
-        if ((rc = ensure_dev(&ws->d_diag, &ws->diag_cap, (size_t)dgp.region_words * (size_t)ctas))) return rc;
+        size_t got = 0;
+        if ((rc = ensure_units(&ws->d_diag, &ws->diag_cap, (size_t)dgp.region_words, (size_t)ctas, 1, &got))) return rc;
+        if (got == 0) {
+            set_error("no device memory for a region of the diagonal kernel");
+            return NO_DIAG_REGION;
+        }
+        ctas = (int)got;
         dgp.region = ws->d_diag;
         dgp.next_item = ws->d_counters;
         dgp.cand_count = ws->d_counters + 1;
@@ -910,8 +949,12 @@ static int run_scan(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int qdbid
                     int do_null3, bool plain, std::vector<std::vector<cmgpu_hit>> &hits_per_win,
                     std::vector<Cand> *cells_out = nullptr, bool calib = false) {
     return host_memory_checked([&]() {
-        return scan_windows(m, ws, semiring, qdbidx, d_dsq, h_dsq, dsq_len, wins, cutoff, do_null3, plain,
-                            hits_per_win, cells_out, calib);
+        auto scan = [&](bool level) {
+            return scan_windows(m, ws, semiring, qdbidx, d_dsq, h_dsq, dsq_len, wins, cutoff, do_null3, plain,
+                                hits_per_win, cells_out, calib, level);
+        };
+        const int rc = scan(false);
+        return rc == NO_DIAG_REGION ? scan(true) : rc;
     });
 }
 

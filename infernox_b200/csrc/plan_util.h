@@ -152,6 +152,18 @@ inline bool node_topology(const cmgpu_cm *cm, std::vector<NodeTopo> &out, const 
     return true;
 }
 
+// The largest of `most`, its halves and `least` that get() says it has had
+// (0: not even the least).  Scratch is sized by the free memory, which another
+// caller may take in between.
+template <class F>
+size_t most_that_fit(size_t most, size_t least, F get) {
+    for (size_t n = std::max(most, least);;) {
+        if (get(n)) return n;
+        if (n <= least) return 0;
+        n = std::max(n / 2, least);
+    }
+}
+
 // A score a floating maximum treats as the reference's `a >= b ? a : b` does
 // in every sum and comparison: not NaN, not +inf, not -0 (with none of these
 // in the tables no sum yields one).

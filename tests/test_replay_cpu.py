@@ -115,3 +115,33 @@ int main() {
 def test_what_an_item_throws_reaches_the_caller(tmp_path):
     r = run(tmp_path, "throws", THROWS)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+FITS = PRELUDE + r"""
+#include "plan_util.h"
+int main() {
+    // the calls made for a limit, and what was had
+    auto tries = [](size_t most, size_t least, size_t limit) {
+        std::vector<size_t> seen;
+        const size_t got = cmx::most_that_fit(most, least, [&](size_t n) {
+            seen.push_back(n);
+            return n <= limit;
+        });
+        seen.push_back(got);
+        return seen;
+    };
+    assert((tries(296, 1, 1000) == std::vector<size_t>{296, 296}));
+    assert((tries(296, 1, 100) == std::vector<size_t>{296, 148, 74, 74}));
+    assert((tries(5, 1, 1) == std::vector<size_t>{5, 2, 1, 1}));
+    assert((tries(5, 1, 0) == std::vector<size_t>{5, 2, 1, 0}));
+    assert((tries(1, 1, 0) == std::vector<size_t>{1, 0}));
+    assert((tries(90, 40, 39) == std::vector<size_t>{90, 45, 40, 0}));
+    assert((tries(30, 40, 40) == std::vector<size_t>{40, 40}));
+    return 0;
+}
+"""
+
+
+def test_scratch_that_fits(tmp_path):
+    r = run(tmp_path, "fits", FITS)
+    assert r.returncode == 0, r.stdout + r.stderr
