@@ -26,6 +26,7 @@ struct DevArena {
         for (Slot &s : slots) cudaFree(s.p);
         slots.clear();
     }
+    size_t held(int slot) const { return slots.size() > (size_t)slot ? slots[slot].cap : 0; }
     template <class T>
     cudaError_t get(int slot, T **out, size_t bytes) {
         if (slots.size() <= (size_t)slot) slots.resize(slot + 1);

@@ -1100,10 +1100,16 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     }
     q->stall_col = -1;
     // room for sixteen reportable cells per column (384 bytes), so that a
-    // window holding a homolog is not scanned twice
+    // window holding a homolog is not scanned twice; within what the buffer
+    // has and a quarter of the free memory, sixteen per window at least
     int64_t columns = 0;
     for (const trq::Win &x : wl) columns += x.j0 - x.i0 + 1;
-    int64_t cap = std::max<int64_t>(4096 + 16 * columns, q->cand_hint);
+    const int64_t least = std::max<int64_t>(4096 + 16 * (int64_t)nw, q->cand_hint);
+    size_t freeb = 0, totalb = 0;
+    TRQ_TRY(cudaMemGetInfo(&freeb, &totalb));
+    int64_t cap = std::min<int64_t>(4096 + 16 * columns,
+                                    (int64_t)((freeb / 4 + ar.held(14)) / sizeof(hb::TrCand)));
+    cap = std::max(cap, least);
     cudaEvent_t ev0, ev1;
     TRQ_TRY(cudaEventCreate(&ev0));
     TRQ_TRY(cudaEventCreate(&ev1));
@@ -1111,7 +1117,13 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     size_t nhc = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
         hb::TrCand *d_c = nullptr;
-        if (ar.get(14, &d_c, sizeof(hb::TrCand) * (size_t)cap)) {
+        cudaError_t e = ar.get(14, &d_c, sizeof(hb::TrCand) * (size_t)cap);
+        if (e == cudaErrorMemoryAllocation && cap > least && attempt == 0) {
+            cudaGetLastError();  // another caller has taken it since
+            cap = least;
+            e = ar.get(14, &d_c, sizeof(hb::TrCand) * (size_t)cap);
+        }
+        if (e != cudaSuccess) {
             cudaEventDestroy(ev0);
             cudaEventDestroy(ev1);
             set_error("truncated QDB scan: device allocation failed");

@@ -2,12 +2,16 @@
 and the same cells."""
 import dataclasses
 
+import numpy as np
 import pytest
 import torch
 
-from infernox_b200 import scan
-from infernox_b200.scan import INSIDE_I32, KERNEL_LEVEL, NOQDB
+from infernox_b200 import _native as N
+from infernox_b200 import model, scan, synth
+from infernox_b200.hb import TrInputs, tr_qdb_scan_batch
+from infernox_b200.scan import CYK_F32, INSIDE_I32, KERNEL_LEVEL, NOQDB
 
+from hb_helpers import tr_tables
 from helpers import frame, models, planted_seq
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +44,28 @@ def test_scan_with_little_device_memory(leave_mb, chunk, kernel):
         torch.cuda.empty_cache()
     assert got == want
     b.close()
+
+
+# 16 reportable cells per column of a 4,000,000-column window would take 1.9 GB.
+def test_truncated_scan_with_little_device_memory():
+    cm = synth.synth_cm("(...)", 1, name="tiny", ins_open=0.005, ins_self=0.1)
+    c = model.configure(cm, local=True)
+    tt = tr_tables(cm, c, 4, True)
+    tri = TrInputs(tt["lmesc"], tt["rmesc"], tt["pty"], tt["lpos"], tt["rpos"], tt["clen"], True,
+                   tt["ilmesc"], tt["irmesc"], tt["ipty"])
+    n = 4000000
+    dsq = frame(synth.random_dsq(n, 0.5, np.random.default_rng(3)))
+    w = np.array([(0, 1, n)], N.WINDOW_DTYPE)
+    res = []
+    for leave_mb in (None, 1200):
+        sc = scan.Scanner(c)
+        held = None
+        if leave_mb:
+            held = torch.empty(torch.cuda.mem_get_info()[0] - (leave_mb << 20), dtype=torch.uint8, device="cuda")
+        try:
+            res.append(tr_qdb_scan_batch(sc, CYK_F32, NOQDB, tri, 4, True, dsq, w, 3.0))
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        sc.close()
+    assert len(res[0][0][0]) > 0 and res[0] == res[1]
