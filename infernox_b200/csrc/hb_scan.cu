@@ -1210,10 +1210,40 @@ int hb_prepare(cmgpu_model *m, HbDev **out) {
 // 3.3 / 7.2, 1,000 - / 6.2 / 8.3, 2,000 14.8 / 11.4 / 9.7; truncated CYK (twice
 // the registers), 40 envelopes 3.0 / 4.5 / 11, 200 5.3 / 5.1 / 14.5, 1,000 - /
 // 19.1 / 22.3, 2,000 37.3 / 35.6 / 32.1.
-int hb_threads(int device, int nenv, bool truncated) {
+int hb_threads(int device, int nenv, bool truncated, bool by_rows) {
     int sms = 148;
+    if (by_rows) return 32;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     return nenv > 10 * sms ? 32 : nenv > (truncated ? 1 : 2) * sms ? 128 : 256;
+}
+
+// What the cell tasks of an envelope come to.  A state's cells are numbered
+// row by row at the width of its widest row, so bands with a few wide rows
+// among narrow ones have numbers without a cell, and each costs a thread a
+// division and a row's load.
+struct CellTasks {
+    int64_t numbers = 0;
+    bool large = false;  // a state's numbers do not fit the kernels' 32 bits
+};
+CellTasks cell_tasks(const hb::State *states, int M) {
+    CellTasks t;
+    for (int v = 0; v < M; v++) {
+        const int64_t n = (int64_t)states[v].nj * states[v].wide;
+        t.numbers += n;
+        t.large = t.large || n > ((int64_t)1 << 30);
+    }
+    return t;
+}
+
+// Whether envelopes [e0, e1) go row by row for that reason: sixteen numbers a
+// cell cost more than the cells themselves.
+bool ragged_rows(const std::vector<CellTasks> &tasks, int32_t e0, int32_t e1, int64_t cells) {
+    int64_t numbers = 0;
+    for (int32_t e = e0; e < e1; e++) {
+        if (tasks[e].large) return true;
+        numbers += tasks[e].numbers;
+    }
+    return numbers / 16 > cells;
 }
 
 int sdelta_h(int st) { return st == MP_ST ? 2 : (st == ML_ST || st == MR_ST || st == IL_ST || st == IR_ST) ? 1 : 0; }
@@ -1353,8 +1383,8 @@ void hb_report(const cmgpu_model *m, const hb::Cand *c, size_t n, const uint8_t 
 int hb_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, int report, int do_null3,
               const uint8_t *dsq_all, int64_t dsq_len, const cmgpu_hb_task *tasks, int32_t e0, int32_t e1,
               const hb::State *st_pin, const hb::Row *row_pin, const std::vector<int64_t> &row_base,
-              const std::vector<int64_t> &alpha_off, cmgpu_hb_result *results, std::vector<cmgpu_hit> &hits,
-              double &ms_total, int &launches) {
+              const std::vector<int64_t> &alpha_off, bool by_rows, cmgpu_hb_result *results,
+              std::vector<cmgpu_hit> &hits, double &ms_total, int &launches) {
     const int n = e1 - e0;
     const int M = m->cm.view.M;
     const int64_t r0 = row_base[e0], nrows = row_base[e1] - r0;
@@ -1388,7 +1418,7 @@ int hb_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, int repor
     hb::Tables t{h->sttype, h->cfirst, h->cnum, h->lev_start, h->lev_states, h->begins, h->tsc, h->oesc,
                  h->endsc, h->beginsc, h->flog, m->cm.view.el_selfsc, h->nlev, h->nbeg,
                  (int)((m->cm.view.flags >> 10) & 1u)};
-    const int threads = hb_threads(m->device, n, false);
+    const int threads = hb_threads(m->device, n, false, by_rows);
     int64_t cap = report ? std::max<int64_t>(4096 + 16 * (int64_t)n, h->cand_hint) : 0;
     cudaEvent_t ev0, ev1;
     HB_TRY(cudaEventCreate(&ev0));
@@ -1487,12 +1517,15 @@ int hb_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int report, i
         return CMGPU_ENOMEM;
     }
     std::vector<std::string> errs(ntask);
+    std::vector<CellTasks> ct(ntask);
     const int nthr = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)std::thread::hardware_concurrency(), 32,
                                                                    (int64_t)ntask / 16 + 1}));
     auto work = [&](int32_t a, int32_t b) {
-        for (int32_t e = a; e < b; e++)
+        for (int32_t e = a; e < b; e++) {
             ncells[e] = fill_envelope(m->cm, tasks[e], dsq_len, dsq_all, st_pin + (size_t)e * M,
                                       row_pin + row_base[e], errs[e]);
+            if (ncells[e] >= 0) ct[e] = cell_tasks(st_pin + (size_t)e * M, M);
+        }
     };
     if (nthr == 1) {
         work(0, ntask);
@@ -1522,7 +1555,8 @@ int hb_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int report, i
         while (e1 < ntask && alpha_off[e1 + 1] - alpha_off[e0] <= budget) e1++;
         rc = host_memory_checked([&]() {
             return hb_launch(m, h, st, semiring, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin, row_pin,
-                             row_base, alpha_off, results, hits, ms, launches);
+                             row_base, alpha_off, ragged_rows(ct, e0, e1, alpha_off[e1] - alpha_off[e0]), results,
+                             hits, ms, launches);
         });
         if (rc) return rc;
         e0 = e1;
@@ -1536,7 +1570,7 @@ int hb_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int report, i
 int tr_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, const hb::TrTab &trt, const TrCtx &cx,
               int report, int do_null3, const uint8_t *dsq_all, int64_t dsq_len, const cmgpu_tr_task *tasks,
               int32_t e0, int32_t e1, const hb::State *st_pin, const hb::Row *row_pin,
-              const std::vector<int64_t> &row_base, const std::vector<int64_t> &alpha_off,
+              const std::vector<int64_t> &row_base, const std::vector<int64_t> &alpha_off, bool by_rows,
               cmgpu_tr_result *results, std::vector<cmgpu_tr_hit> &hits, double &ms_total, int &launches) {
     const int n = e1 - e0;
     const int M = m->cm.view.M;
@@ -1571,7 +1605,7 @@ int tr_launch(cmgpu_model *m, HbDev *h, cudaStream_t st, int semiring, const hb:
     hb::Tables t{h->sttype, h->cfirst, h->cnum, h->lev_start, h->lev_states, h->begins, h->tsc, h->oesc,
                  h->endsc, h->beginsc, h->flog, m->cm.view.el_selfsc, h->nlev, h->nbeg,
                  (int)((m->cm.view.flags >> 10) & 1u)};
-    const int threads = hb_threads(m->device, n, true);
+    const int threads = hb_threads(m->device, n, true, by_rows);
     int64_t cap = report ? std::max<int64_t>(4096 + 16 * (int64_t)n, h->tr_cand_hint) : 0;
     cudaEvent_t ev0, ev1;
     HB_TRY(cudaEventCreate(&ev0));
@@ -1683,6 +1717,7 @@ int tr_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, const cmgpu_t
         return CMGPU_ENOMEM;
     }
     std::vector<std::string> errs(ntask);
+    std::vector<CellTasks> ct(ntask);
     const int nthr = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)std::thread::hardware_concurrency(), 32,
                                                                    (int64_t)ntask / 16 + 1}));
     auto work = [&](int32_t a, int32_t b) {
@@ -1696,6 +1731,7 @@ int tr_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, const cmgpu_t
                 for (int v = 0; v < M; v++)
                     sp[v].pad = (tk.jvalid[v] ? 1 : 0) | (tk.lvalid[v] ? 2 : 0) | (tk.rvalid[v] ? 4 : 0) |
                                 (tk.tvalid[v] ? 8 : 0);
+            if (ncells[e] >= 0) ct[e] = cell_tasks(sp, M);
         }
     };
     if (nthr == 1) {
@@ -1747,7 +1783,8 @@ int tr_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, const cmgpu_t
         while (e1 < ntask && alpha_off[e1 + 1] - alpha_off[e0] <= budget) e1++;
         rc = host_memory_checked([&]() {
             return tr_launch(m, h, st, semiring, trt, cx, report, do_null3, dsq_all, dsq_len, tasks, e0, e1, st_pin,
-                             row_pin, row_base, alpha_off, results, hits, ms, launches);
+                             row_pin, row_base, alpha_off, ragged_rows(ct, e0, e1, alpha_off[e1] - alpha_off[e0]),
+                             results, hits, ms, launches);
         });
         if (rc) return rc;
         e0 = e1;

@@ -15,10 +15,10 @@ import torch
 import oracle
 from infernox_b200 import _native as N
 from infernox_b200 import model, synth
-from infernox_b200.hb import (TrInputs, hb_scan_batch, ref_itr_inside_scan, ref_tr_cyk_scan, tr_scan_hb_batch)
+from infernox_b200.hb import (Bands, TrInputs, hb_scan_batch, ref_itr_inside_scan, ref_tr_cyk_scan, tr_scan_hb_batch)
 from infernox_b200.scan import CYK_F32, INSIDE_I32, NOQDB, QDB1, QDB2, Scanner
 
-from hb_helpers import ragged_bands, rect_bands, tr_tables, tr_valid, truncated_window
+from hb_helpers import as_tuple, ragged_bands, rect_bands, tr_tables, tr_valid, truncated_window
 from helpers import frame, models, oracle_cfg, planted_seq
 
 pytestmark = pytest.mark.gpu
@@ -132,4 +132,38 @@ def test_truncated_scan_of_tiny_models(ss, loc, qdb):
             assert bits(go[1]) == bits(ro[1]) and go[2] == ro[2] and bits(go[3]) == bits(ro[3])
             assert [(a, b, bits(s), bits(e), m, r) for a, b, s, e, m, r in go[0]] == \
                    [(a, b, bits(s), bits(e), m, r) for a, b, s, e, m, r in ro[0]]
+    sc.close()
+
+
+# One row of 31,000 spans among 70,000 rows of one: 70,000 x 31,000 cell numbers
+# of a state do not fit 32 bits.  (200: sixteen numbers a cell and more.)
+@pytest.mark.parametrize("truncated", [False, True])
+@pytest.mark.parametrize("rows,wide", [(700, 200), (70000, 31000)])
+def test_hmm_banded_one_wide_row(rows, wide, truncated):
+    cm, _, l = models("small0")
+    sc = Scanner(l)
+    rng = np.random.default_rng(rows)
+    dsq = frame(rng.integers(0, 4, rows).astype(np.uint8))
+    mins, maxs = [], []
+    for v in range(l.M):
+        lo = np.full(rows if v < 12 else 100, 0 if l.sttype[v] == 7 else 1, np.int32)  # v < 12: the first nodes
+        hi = lo.copy()
+        if l.sttype[v] != 7:
+            hi[1:] = 2
+            if v < 12 and l.sttype[v] != 5:  # (an IR state's diagonals would pass every row)
+                hi[wide + 100] = wide
+        mins.append(lo)
+        maxs.append(hi)
+    bands = Bands.from_rows(np.full(l.M, 1), np.array([len(x) for x in mins]), mins, maxs)
+    if truncated:
+        tt = tr_tables(cm, l, 4, True)
+        valid = tr_valid(l.M, 1, 4, True)
+        ro = oracle.tr_hb_scan(l, False, tt, valid, as_tuple(bands), dsq, 1, rows, -6.0, True, 4, -1e30, True)
+        go = tr_scan_hb_batch(sc, N.CYK_F32, TrInputs(tt["lmesc"], tt["rmesc"], tt["pty"], tt["lpos"], tt["rpos"],
+                                                      tt["clen"], True), 4, True, dsq,
+                              [(0, 1, rows, -1e30, -6.0, bands, valid)])[0]
+    else:
+        ro = oracle.hb_scan(l, False, as_tuple(bands), dsq, 1, rows, -1e30, True, -6.0, True)
+        go = hb_scan_batch(sc, N.CYK_F32, True, True, dsq, [(0, 1, rows, -1e30, -6.0, bands)])[0]
+    assert same(go, ro)
     sc.close()
