@@ -495,9 +495,9 @@ int cmgpu_tr_scan_hb_batch(const cmgpu_model *m, void *stream, int semiring, con
  * ref_itr_inside_scan (CMGPU_INSIDE_I32, :226) of residues i0..j0 with the
  * QDB bands qdbidx (CMGPU_NOQDB / QDB1 / QDB2) in pass pass_idx: the hits
  * after overlap removal, vsc_root and its mode, and the best score spanning
- * the full window as the reference computes it (bsc_full).  The scan runs
- * the columns of a window in order on one CTA: its ROOT row carries over
- * from column to column as in the reference, so windows are not split. */
+ * the full window as the reference computes it (bsc_full).  One CTA scans a
+ * window: its ROOT row carries over from column to column as in the
+ * reference, so windows are not split. */
 typedef struct cmgpu_trq_result {
     float vsc_root;
     int32_t vmode;
@@ -518,13 +518,25 @@ int cmgpu_tr_qdb_scan_batch(const cmgpu_model *m, void *stream, int semiring, in
 /* Test hook for failure detection: in the next truncated QDB call the warp
  * that runs column `column` (0-based within each window) never publishes its
  * progress, so the next column's bounded wait runs out (about a second) and
- * the call fails with CMGPU_ETIMEOUT instead of hanging; -1 clears it.  The
- * model stays usable. */
+ * the call fails with CMGPU_ETIMEOUT instead of hanging; -1 clears it.  That
+ * call runs CMGPU_TRQ_WAVEFRONT.  The model stays usable. */
 int cmgpu_tr_qdb_inject_stall(cmgpu_model *m, int32_t column);
 /* Device memory the truncated QDB scan may hold in window decks at once
  * (each resident window has its own; the grid is cut to fit).  0 restores
  * the default, 4 GiB. */
 int cmgpu_tr_qdb_set_deck_budget(cmgpu_model *m, int64_t bytes);
+/* Kernels of the truncated QDB scan; both give the same results.  DIAG walks
+ * the diagonals and takes every model whose nodes are laid out as the
+ * reference's model builder lays them out and whose scores are plain (no NaN,
+ * +inf or -0; sums of integer scores below 16,000 bits); WAVEFRONT walks the
+ * columns and takes any model.  AUTO is DIAG where it applies. */
+#define CMGPU_TRQ_AUTO 0
+#define CMGPU_TRQ_WAVEFRONT 1
+#define CMGPU_TRQ_DIAG 2 /* what AUTO runs; reported only */
+/* CMGPU_TRQ_AUTO or CMGPU_TRQ_WAVEFRONT for the model's next calls. */
+int cmgpu_tr_qdb_set_kernel(cmgpu_model *m, int kernel);
+/* The kernel of the model's last truncated QDB call (0: none yet). */
+int cmgpu_tr_qdb_kernel(const cmgpu_model *m, int32_t *used);
 /* Device time, J-plane cells and launches of the last truncated QDB call. */
 int cmgpu_tr_qdb_stats(const cmgpu_model *m, double *kernel_ms, int64_t *cells, int32_t *launches);
 

@@ -83,6 +83,7 @@ struct TrqDev {
     double last_ms = 0;
     int64_t last_cells = 0;
     int32_t last_launches = 0;
+    int32_t kernel = CMGPU_TRQ_AUTO, last_kernel = 0;
     int32_t stall_col = -1;  // test hook: this column never publishes its progress (next call only)
     int64_t deck_budget = (int64_t)4 << 30;  // bytes of decks resident at once (bounds the grid)
 };
@@ -931,14 +932,14 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     TRQ_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
     const int64_t budget = q->deck_budget;  // bytes of decks
 
-    // The diagonal kernel takes every model with cm_from_guide's node layout;
-    // the column wavefront takes the others, and the calls of the test hook,
-    // which stalls one of its columns.
+    // The diagonal kernel takes every model with cm_from_guide's node layout
+    // and plain scores; the column wavefront takes the others, the calls that
+    // ask for it, and those of the test hook, which stalls one of its columns.
     std::vector<trqd::Node> nodes;
     trqd::Params dgp{};
     std::vector<char> skip(M, 0);
     for (int v = 1; v < M; v++) skip[v] = q->kind_h[v] == trq::K_SKIP;
-    const bool diag = q->stall_col < 0 &&
+    const bool diag = q->stall_col < 0 && q->kernel == CMGPU_TRQ_AUTO &&
                       trqd::build(&c.view, ins, dxcap, skip, pty, pbeg, lm, rm, base, q->begl_h, q->esc_plain,
                                   q->esc_best, nodes, &dgp.nbif);
     std::vector<int2> units, il_units;
@@ -1099,6 +1100,7 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
                            nl, NC, nstep, q->stall_col};
     }
     q->stall_col = -1;
+    q->last_kernel = diag ? CMGPU_TRQ_DIAG : CMGPU_TRQ_WAVEFRONT;
     // room for sixteen reportable cells per column (384 bytes), so that a
     // window holding a homolog is not scanned twice; within what the buffer
     // has and a quarter of the free memory, sixteen per window at least
@@ -1272,6 +1274,21 @@ extern "C" int cmgpu_tr_qdb_set_deck_budget(cmgpu_model *m, int64_t bytes) {
     int rc = trq_prepare(m, &q);
     if (rc) return rc;
     q->deck_budget = bytes > 0 ? bytes : ((int64_t)4 << 30);
+    return CMGPU_OK;
+}
+
+extern "C" int cmgpu_tr_qdb_set_kernel(cmgpu_model *m, int kernel) {
+    if (!m || (kernel != CMGPU_TRQ_AUTO && kernel != CMGPU_TRQ_WAVEFRONT)) return CMGPU_EINVAL;
+    TrqDev *q = nullptr;
+    int rc = trq_prepare(m, &q);
+    if (rc) return rc;
+    q->kernel = kernel;
+    return CMGPU_OK;
+}
+
+extern "C" int cmgpu_tr_qdb_kernel(const cmgpu_model *m, int32_t *used) {
+    if (!m || !used) return CMGPU_EINVAL;
+    *used = m->trq ? m->trq->last_kernel : 0;
     return CMGPU_OK;
 }
 

@@ -373,6 +373,21 @@ def tr_qdb_stats(sc: Scanner):
     return ms.value, cells.value, launches.value
 
 
+TRQ_AUTO, TRQ_WAVEFRONT, TRQ_DIAG = 0, 1, 2  # kernels of the truncated QDB scan (CMGPU_TRQ_*)
+
+
+def tr_qdb_set_kernel(sc: Scanner, kernel: int) -> None:
+    """TRQ_AUTO or TRQ_WAVEFRONT for this model's next truncated QDB calls."""
+    N.check(N.lib().cmgpu_tr_qdb_set_kernel(sc._model, kernel))
+
+
+def tr_qdb_kernel(sc: Scanner) -> int:
+    """The kernel of this model's last truncated QDB call (0: none yet)."""
+    used = C.c_int32()
+    N.check(N.lib().cmgpu_tr_qdb_kernel(sc._model, C.byref(used)))
+    return used.value
+
+
 # row of the truncated-begin penalties a pass uses (pty_idx_for_pass,
 # src/cm_trunc.rs:99-107): 5'-and-3' (forced or any), 5'-only, 3'-only
 PTY_ROW = {2: 1, 3: 2, 4: 0, 5: 0}
