@@ -117,7 +117,7 @@ def test_bands_without_short_spans_match_oracle(name, sr, band):
     up = {k: np.where(np.asarray(ref.sttype) == 7, getattr(ref, k), np.maximum(getattr(ref, k), 5)).astype(np.int32)
           for k in ("dmin1", "dmin2")}
     up.update({k: np.maximum(getattr(ref, k), up["dmin" + k[-1]]).astype(np.int32) for k in ("dmax1", "dmax2")})
-    c = dataclasses.replace(ref, **up)
+    c = dataclasses.replace(ref, **up, _struct=None)
     s = scan.Scanner(c)
     for n in (40, 700):
         dsq = frame(seq_of(cm, n, 3 * n))

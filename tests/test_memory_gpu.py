@@ -25,7 +25,7 @@ DIAG = 3  # CMGPU_KERNEL_DIAG in the statistics
 @pytest.mark.parametrize("leave_mb,chunk,kernel", [(560, 0, KERNEL_LEVEL), (1500, 100, DIAG)])
 def test_scan_with_little_device_memory(leave_mb, chunk, kernel):
     cm, _, l = models("mb3")
-    c = dataclasses.replace(l, W=6000)
+    c = dataclasses.replace(l, W=6000, _struct=None)
     dsq = frame(planted_seq(cm, 300, 0.5, 1, seed=4))
     a = scan.Scanner(c)
     a.set_shape(0, 0, chunk, 0)
