@@ -231,6 +231,12 @@ int cmgpu_workspace_set_shape(cmgpu_workspace *ws, int ctas_per_sm, int threads,
  * CMGPU_EINVAL.  With SWEEP, set_shape's `lanes` is the warps per CTA (1..12)
  * and `chunk` the residues per work item. */
 int cmgpu_workspace_set_kernel(cmgpu_workspace *ws, int kernel);
+/* Test hook for failure detection: in the workspace's next scan on the
+ * diagonal kernel (CMGPU_KERNEL_DIAG) with an item of more than 32 columns,
+ * the first wait of a warp for its neighbour runs out (two seconds), every
+ * other wait gives up, and the call fails with CMGPU_ETIMEOUT instead of
+ * hanging.  The workspace stays usable. */
+int cmgpu_workspace_inject_stall(cmgpu_workspace *ws);
 
 /* ---- scanner entry points ----------------------------------------------- */
 

@@ -92,6 +92,7 @@ struct cmgpu_workspace {
     int chunk = 0;        // 0 = auto
     int lanes = 0;        // 0 = tuned
     int kernel = 0;       // CMGPU_KERNEL_*
+    bool stall = false;   // test hook: the next diagonal scan's waits run out
     int sm_count = 148;
     cmgpu_stats stats{};
     ~cmgpu_workspace() {
@@ -716,6 +717,8 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
         // the instruction cache decides (296 windows of 512: 32 ms at a slack
         // of 2, 49 at 8), with idle SMs the handshake does (one window of 256:
         // 10.2 ms at 2, 8.8 at 8).
+        dgp.stall = ws->stall ? 1 << 24 : 0;
+        ws->stall = false;
         dgp.slack = (int64_t)items.size() >= (int64_t)ws->sm_count * best_c / 2 ? 2 : DG_XCH;
         // the regions stay within half of the free device memory
         size_t freeb = 0, totalb = 0;
@@ -1065,6 +1068,12 @@ int cmgpu_workspace_stats(const cmgpu_workspace *ws, cmgpu_stats *out) {
 int cmgpu_workspace_set_kernel(cmgpu_workspace *ws, int kernel) {
     if (!ws || kernel < CMGPU_KERNEL_AUTO || kernel > CMGPU_KERNEL_SWEEP) return CMGPU_EINVAL;
     ws->kernel = kernel;
+    return CMGPU_OK;
+}
+
+int cmgpu_workspace_inject_stall(cmgpu_workspace *ws) {
+    if (!ws) return CMGPU_EINVAL;
+    ws->stall = true;
     return CMGPU_OK;
 }
 

@@ -72,6 +72,7 @@ struct DgParams {
     int nnodes;
     const uint32_t *tsc, *endsc, *esc, *el_sca, *bsv;
     int slack;                   // steps a warp may be ahead of its right neighbour
+    int stall;                   // 0, or (test hook) steps more than the right neighbour will ever do
     int W, ring_cols, ring_len;  // ring_len: residues kept per CTA (power of two)
     int root_dn, root_dxcap;
     int inside, local, begin_key, prefilter, do_null3;

@@ -80,7 +80,7 @@ struct DgCtx {
 };
 
 // Waits between warps: each warp publishes how many steps it has finished.
-constexpr int DG_TRIES = 1 << 24;  // polls before a wait gives up (a second or so)
+constexpr int DG_TRIES = 1 << 24;  // polls before a wait gives up (two seconds or so)
 
 __device__ __forceinline__ int dg_seen(uint32_t addr) {
     int v;
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             // models is the one ROOT still reads its child from (and a group of
             // fewer steps than the slack would let a warp run two ahead).  About
             // a step of waiting per group of a thousand.
-            if (c.w < c.nw - 1) dg_wait(c, c.w + 1, c.step);
+            if (c.w < c.nw - 1) dg_wait(c, c.w + 1, c.step + p.stall);
             c.first = g0 == 0;
             c.last = g0 + cols >= c.ncols;
             c.jrel = g0 + c.col;

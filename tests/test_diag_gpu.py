@@ -4,6 +4,7 @@ partial group, windows shorter than W, forced pieces -- against the oracle
 bit for bit, and every ROOT cell against the level kernel over all semirings,
 band sets and configurations."""
 import dataclasses
+import time
 
 import numpy as np
 import pytest
@@ -143,3 +144,24 @@ def test_tiny_models_match_level_kernel(ss, local, sr, band):
         ca, cb = a.scan_cells(sr, band, dsq, 1, n, -500.0), b.scan_cells(sr, band, dsq, 1, n, -500.0)
         assert (a.stats()["kernel"], b.stats()["kernel"]) == (DIAG, KERNEL_LEVEL)
         assert len(ca) > n and ca == cb
+
+
+# Failure detection without a GPU fault: a warp waits for a step that its
+# neighbour never reaches, gives up, and so does every other wait; the same
+# workspace then scans correctly.
+@pytest.mark.parametrize("n", [100, 3000])
+@pytest.mark.parametrize("sr,band", [(CYK_F32, QDB1), (INSIDE_I32, NOQDB)])
+def test_waits_of_the_diagonal_scan_run_out(sr, band, n):
+    cm, _, l = models("small2")
+    s = scan.Scanner(l)
+    s.set_shape(0, 0, 1152, 0)
+    dsq = frame(seq_of(cm, n, 70 + n))
+    want, _, _, _ = oracle.qdb_scan(oracle_cfg("small2", True), sr, band, dsq, 1, n, -20.0, True)
+    for _ in range(2):
+        N.check(N.lib().cmgpu_workspace_inject_stall(s._ws))
+        t0 = time.perf_counter()
+        with pytest.raises(N.CmgpuError, match="timed out") as ei:
+            s.generic_scan(sr, band, dsq, 1, n, -20.0, True)
+        assert ei.value.rc == N.CMGPU_ETIMEOUT and time.perf_counter() - t0 < 30
+        assert bits(s.generic_scan(sr, band, dsq, 1, n, -20.0, True)) == bits(want)
+        assert s.stats()["kernel"] == DIAG
