@@ -223,7 +223,10 @@ void cmgpu_workspace_free(cmgpu_workspace *ws);
 int cmgpu_workspace_stats(const cmgpu_workspace *ws, cmgpu_stats *out);
 /* Launch shape override for tuning (0 keeps the tuned value): CTAs per SM
  * (1..4), threads in {128,256,512}, residues per work item, work items
- * scanned side by side per CTA (1..8). */
+ * scanned side by side per CTA (1..16).  CMGPU_KERNEL_DIAG, which AUTO runs,
+ * takes one item per CTA and as many warps as the items are long, so there
+ * only the CTAs per SM (at most) and the residues per item act; `threads` and
+ * `lanes` are for CMGPU_KERNEL_LEVEL. */
 int cmgpu_workspace_set_shape(cmgpu_workspace *ws, int ctas_per_sm, int threads, int chunk,
                               int lanes);
 /* Kernel choice for the scans of this workspace (CMGPU_KERNEL_*).  A scan

@@ -25,6 +25,7 @@ CMGPU_ENOSPACE = -7
 CYK_F32, INSIDE_I32, INSIDE_F32 = 0, 1, 2
 NOQDB, QDB1, QDB2 = 0, 1, 2
 KERNEL_AUTO, KERNEL_LEVEL, KERNEL_SWEEP = 0, 1, 2
+KERNEL_DIAG = 3  # what AUTO runs; reported in the statistics only
 
 P = C.POINTER
 

@@ -668,7 +668,7 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
             return CMGPU_EDEVICE;
         }
         best_c = ws->ctas_per_sm > 0 ? std::min(ws->ctas_per_sm, occ) : occ;
-        ws->stats.lanes = best_l;
+        ws->stats.lanes = 1;
     }
 
     if ((rc = ensure_dev(&ws->d_items, &ws->items_cap, items.size()))) return rc;

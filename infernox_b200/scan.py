@@ -104,7 +104,8 @@ class Scanner:
         N.check(N.lib().cmgpu_workspace_set_shape(self._ws, ctas_per_sm, threads, chunk, lanes))
 
     def set_kernel(self, kernel: int) -> None:
-        """KERNEL_AUTO, KERNEL_LEVEL (CTA level schedule) or KERNEL_SWEEP (warp node sweep)."""
+        """KERNEL_AUTO (the diagonal kernel wherever it applies, else the level kernel),
+        KERNEL_LEVEL (CTA level schedule) or KERNEL_SWEEP (warp node sweep)."""
         N.check(N.lib().cmgpu_workspace_set_kernel(self._ws, kernel))
 
     def autotune(self, semiring: int, qdbidx: int, buf: np.ndarray, windows: np.ndarray,
@@ -114,22 +115,24 @@ class Scanner:
         pieces repeat fewer W-1 warm-up columns, shorter ones balance the
         tail) for this model and batch by timing one scan per candidate; the
         fastest stays set on this Scanner.  Every candidate returns the same
-        hits (checked)."""
+        hits (checked).  The diagonal kernel takes its own lanes and threads:
+        where that one runs, only the item lengths are tried."""
         best, ref, trials = None, None, []
-        for th in threads:
-            for ln in lanes:
-                for cw in chunks_w:
-                    chunk = int(cw * self.cm.W)
-                    self.set_shape(0, th, chunk, ln)
-                    hits = self.scan_batch(semiring, qdbidx, buf, windows, cutoff, False, device_buf=device_buf)
-                    ms = self.stats()["kernel_ms"]
-                    if ref is None:
-                        ref = hits
-                    elif not np.array_equal(hits, ref):
-                        raise RuntimeError("launch shapes disagree")
-                    trials.append({"lanes": ln, "threads": th, "chunk": chunk, "kernel_ms": ms})
-                    if best is None or ms < best["kernel_ms"]:
-                        best = trials[-1]
+        for th, ln in [(th, ln) for th in threads for ln in lanes]:
+            if trials and self.stats()["kernel"] == N.KERNEL_DIAG:
+                break
+            for cw in chunks_w:
+                chunk = int(cw * self.cm.W)
+                self.set_shape(0, th, chunk, ln)
+                hits = self.scan_batch(semiring, qdbidx, buf, windows, cutoff, False, device_buf=device_buf)
+                ms = self.stats()["kernel_ms"]
+                if ref is None:
+                    ref = hits
+                elif not np.array_equal(hits, ref):
+                    raise RuntimeError("launch shapes disagree")
+                trials.append({"lanes": ln, "threads": th, "chunk": chunk, "kernel_ms": ms})
+                if best is None or ms < best["kernel_ms"]:
+                    best = trials[-1]
         self.set_shape(0, best["threads"], best["chunk"], best["lanes"])
         return {"best": best, "trials": trials}
 

@@ -165,3 +165,16 @@ def test_waits_of_the_diagonal_scan_run_out(sr, band, n):
         assert ei.value.rc == N.CMGPU_ETIMEOUT and time.perf_counter() - t0 < 30
         assert bits(s.generic_scan(sr, band, dsq, 1, n, -20.0, True)) == bits(want)
         assert s.stats()["kernel"] == DIAG
+
+
+def test_autotune_tries_what_acts():
+    cm, _, l = models("small2")
+    dsq = frame(seq_of(cm, 2000, 5))
+    w = np.array([(0, 1, 2000), (0, 300, 900)], N.WINDOW_DTYPE)
+    s = scan.Scanner(l)
+    t = s.autotune(INSIDE_I32, NOQDB, dsq, w, 5.0, chunks_w=(0, 4))
+    assert s.stats()["kernel"] == DIAG and s.stats()["lanes"] == 1  # work items per CTA
+    assert [x["chunk"] for x in t["trials"]] == [0, 4 * l.W]
+    s.set_kernel(KERNEL_LEVEL)
+    t = s.autotune(INSIDE_I32, NOQDB, dsq, w, 5.0, lanes=(1, 2), chunks_w=(0, 4))
+    assert len(t["trials"]) == 4
