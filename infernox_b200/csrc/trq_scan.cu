@@ -1107,10 +1107,12 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
     int64_t columns = 0;
     for (const trq::Win &x : wl) columns += x.j0 - x.i0 + 1;
     const int64_t least = std::max<int64_t>(4096 + 16 * (int64_t)nw, q->cand_hint);
-    size_t freeb = 0, totalb = 0;
-    TRQ_TRY(cudaMemGetInfo(&freeb, &totalb));
-    int64_t cap = std::min<int64_t>(4096 + 16 * columns,
-                                    (int64_t)((freeb / 4 + ar.held(14)) / sizeof(hb::TrCand)));
+    int64_t cap = 4096 + 16 * columns;
+    if ((size_t)cap * sizeof(hb::TrCand) > ar.held(14)) {
+        size_t freeb = 0, totalb = 0;
+        TRQ_TRY(cudaMemGetInfo(&freeb, &totalb));
+        cap = std::min<int64_t>(cap, (int64_t)((freeb / 4 + ar.held(14)) / sizeof(hb::TrCand)));
+    }
     cap = std::max(cap, least);
     cudaEvent_t ev0, ev1;
     TRQ_TRY(cudaEventCreate(&ev0));
