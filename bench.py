@@ -72,6 +72,11 @@ CUTOFF_BITS = 15.0                # stands in for the E-value threshold
 # roofline's traffic is this times the cells of a launch
 TRAFFIC_B_PER_CELL = {("level", 1, 0): 13.59}
 
+# The oracle, a C port of the reference's scanners, is timed as `cpu_baseline`;
+# it is not the reference.
+REFERENCE_UNAVAILABLE = ("the reference is a Rust crate: no cargo or rustc here, its crates are not vendored, and "
+                         "there is no network")
+
 
 def env_rank():
     return (int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1)),
@@ -320,6 +325,10 @@ def main():
     ap.add_argument("--plain-windows", type=int, default=16)
     ap.add_argument("--envelopes", type=int, default=2000, help="envelopes per step (HB workloads)")
     args = ap.parse_args()
+    if args.impl == "reference":
+        if env_rank()[0] == 0:
+            print(json.dumps({"impl": "reference", "unavailable": REFERENCE_UNAVAILABLE}))
+        return
     if args.workload in FILTER_WORKLOADS:
         return filter_main(args)
     if args.workload == "serve":
@@ -356,30 +365,6 @@ def main():
               "homologs": f"{PLANT_FRACTION:.0%} of the sequences carry one homolog sampled from the model",
               "parallelism": f"dp{world}: cost-balanced window split, hits gathered to rank 0",
               "l2": "flushed (256 MB write) before each timed step"}
-
-    if args.impl == "reference":
-        if rank != 0:
-            return
-        per_step = max(2.0, args.cpu_seconds / max(1, args.steps))
-        for _ in range(args.warmup):
-            cpu_baseline(cm, w, buf, [tuple(x) for x in wins], per_step)
-        samples = [cpu_baseline(cm, w, buf, [tuple(x) for x in wins], per_step) for _ in range(args.steps)]
-        cells, secs = sum(x["cells"] for x in samples), sum(x["seconds"] for x in samples)
-        rate = sum(x["value"] * x["seconds"] for x in samples) / secs
-        cb = {"value": rate, "unit": "Gcells/s", "cores": samples[0]["cores"], "kind": "port",
-              "build": samples[0]["build"],
-              "sample": f"{args.steps} steps of about {per_step:.1f} s, each a seeded random sample of the "
-                        f"batch's windows of every length on {samples[0]['cores']} threads (after "
-                        f"{args.warmup} warm-up samples); rate = sum of the threads' own rates"}
-        line = {"impl": "reference", "metric": "CYK/Inside scan Gcells/s", "value": cb["value"],
-                "unit": "Gcells/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
-                "ms_per_step": 1e3 * secs / max(1, args.steps),
-                "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32",
-                "data": "synthetic", "config": config, "cpu_baseline": cb,
-                "e2e": {"value": cb["value"], "unit": "Gcells/s", "h2d_bytes_per_step": 0,
-                        "d2h_bytes_per_step": 0}}
-        print(json.dumps(line))
-        return
 
     import torch
     torch.cuda.set_device(local_rank)
@@ -810,27 +795,6 @@ def filter_main(args):
                 "sample": f"{st['n']} of {len(units)} units of one step's inputs, {dt:.1f} s on {cores} threads",
                 "cells": st["cells"], "seconds": dt}
 
-    if args.impl == "reference":
-        if rank != 0:
-            return
-        per_step = max(1.0, args.cpu_seconds / max(1, args.steps))
-        for _ in range(args.warmup):
-            cpu_sample(per_step)
-        samples = [cpu_sample(per_step) for _ in range(args.steps)]
-        cells, secs = sum(x["cells"] for x in samples), sum(x["seconds"] for x in samples)
-        val = cells / secs / div
-        cb = {"value": val, "unit": unit, "cores": cores, "kind": "port",
-              "sample": f"{args.steps} steps of {per_step:.1f} s, each a bounded sample of one step's units "
-                        f"on {cores} threads (after {args.warmup} warm-up samples)"}
-        print(json.dumps({"impl": "reference", "metric": FILTER_METRIC[kind], "value": val, "unit": unit,
-                          "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
-                          "ms_per_step": 1e3 * secs / max(1, args.steps), "higher_is_better": True,
-                          "scaling": "weak", "vs_baseline": None, "dtype": FILTER_DTYPE[kind], "data": "synthetic",
-                          "config": config, "cpu_baseline": cb,
-                          "e2e": {"value": val, "unit": unit, "h2d_bytes_per_step": 0,
-                                  "d2h_bytes_per_step": 0}}))
-        return
-
     import torch
     torch.cuda.set_device(local_rank)
     stream = torch.cuda.current_stream()
@@ -989,39 +953,6 @@ def serve_main(args):
               "cutoffs_bits": {"f6": 12.0, "final": CUTOFF_BITS, "note": "bit cutoffs stand in for the "
                                "E-value thresholds (no calibration)"},
               "residues": int(sum(r.residues for r in reqs)), "library_build_s": round(t_build, 1)}
-    if args.impl == "reference":
-        # the oracle on the host cores: the per-query, per-model loop of cmscan
-        # on a bounded sample (the first requests, all models), one thread per model
-        oracle = _oracle()
-        from concurrent.futures import ThreadPoolExecutor
-        from infernox_b200.synth import revcomp
-        cores = os.cpu_count() or 1
-        sample = sorted(reqs, key=lambda r: len(r.seq))[: max(1, min(args.steps, 4))]
-
-        def one(k_req):
-            k, r = k_req
-            for s in (r.seq, revcomp(r.seq)):
-                dsq = np.concatenate([[255], s, [255]]).astype(np.uint8)
-                envs = oracle.cyk_seq_filter(cfgs[k], dsq, len(s), 12.0, True)
-                if envs:
-                    oracle.final_stage_inside_opt(cfgs[k], dsq, envs, CUTOFF_BITS, True, False)
-
-        t0 = time.perf_counter()
-        with ThreadPoolExecutor(cores) as ex:
-            list(ex.map(one, [(k, r) for r in sample for k in range(len(cfgs))]))
-        dt = time.perf_counter() - t0
-        value = len(sample) / dt
-        line = {"impl": "reference", "metric": "served sequences/s (cmscan --nohmm, CM library)", "value": value,
-                "unit": "seq/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
-                "ms_per_step": 1e3 * dt / max(1, len(sample)), "higher_is_better": True, "scaling": "weak",
-                "vs_baseline": None, "dtype": "f32+int32", "data": "synthetic", "config": config,
-                "cpu_baseline": {"value": value, "unit": "seq/s", "cores": cores, "kind": "port",
-                                 "sample": f"the {len(sample)} shortest queries ({sum(len(r.seq) for r in sample)} nt) "
-                                           f"against all {len(cfgs)} models, threads over models"},
-                "e2e": {"value": value, "unit": "seq/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-        print(json.dumps(line))
-        return
-
     import torch
     torch.cuda.set_device(local_rank)
     srv = serve.Server(cfgs, device=local_rank, budget_residues=args.serve_budget)
@@ -1178,27 +1109,6 @@ def calibrate_main(args):
                 "cells": st["cells"], "seconds": dt}
 
     metric = "cmcalibrate scan Gcells/s (4 exp modes, bit-exact)"
-    if args.impl == "reference":
-        if rank != 0:
-            return
-        per_step = max(1.0, args.cpu_seconds / max(1, args.steps))
-        for _ in range(args.warmup):
-            cpu_sample(per_step)
-        samples = [cpu_sample(per_step) for _ in range(args.steps)]
-        cells, secs = sum(x["cells"] for x in samples), sum(x["seconds"] for x in samples)
-        val = cells / secs / 1e9
-        cb = {"value": val, "unit": "Gcells/s", "cores": cores, "kind": "port",
-              "sample": f"{args.steps} steps of {per_step:.1f} s, each a bounded sample of one calibration's "
-                        f"(sequence, mode) scans on {cores} threads"}
-        print(json.dumps({"impl": "reference", "metric": metric, "value": val, "unit": "Gcells/s",
-                          "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
-                          "ms_per_step": 1e3 * secs / max(1, args.steps), "higher_is_better": True,
-                          "scaling": "weak", "vs_baseline": None, "dtype": "f32/int32", "data": "synthetic",
-                          "config": config, "cpu_baseline": cb,
-                          "e2e": {"value": val, "unit": "Gcells/s", "h2d_bytes_per_step": 0,
-                                  "d2h_bytes_per_step": 0}}))
-        return
-
     import torch
     dist = None
     if world > 1:
