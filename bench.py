@@ -66,11 +66,13 @@ FILTER_WORKLOADS = ("f1-ssv", "f2-vit", "f3-fwd", "f3-cascade", "hb-cyk", "hb-in
 OPS_PER_TERM = {0: 2.0, 1: 7.0}   # CYK: FADD + select; Inside: 6 INT + 1 LDS
 OPS_PER_CELL = 2.0                # emission add + store
 CUTOFF_BITS = 15.0                # stands in for the E-value threshold
-# DRAM bytes (read + write) per DP cell of the scan kernel, from one ncu
-# capture of this bench's default step (profiles/qdb_scan_inside_nonbanded_
-# traffic.txt: 1.438e12 bytes over 1.058e11 cells in one launch); the
+# DRAM bytes (read + write) per DP cell of the scan kernels, from one ncu
+# capture each: level, this bench's default step (profiles/qdb_scan_inside_
+# nonbanded_traffic.txt: 1.438e12 bytes over 1.058e11 cells in one launch);
+# diagonal, 296 windows of 512 residues of the same model (profiles/
+# diag_scan_inside_nonbanded.txt: 5.572e10 bytes over 7.199e9 cells).  The
 # roofline's traffic is this times the cells of a launch
-TRAFFIC_B_PER_CELL = {("level", 1, 0): 13.59}
+TRAFFIC_B_PER_CELL = {("level", 1, 0): 13.59, ("diagonal", 1, 0): 7.74}
 
 # The oracle, a C port of the reference's scanners, is timed as `cpu_baseline`;
 # it is not the reference.
