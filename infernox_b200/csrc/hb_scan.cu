@@ -1502,6 +1502,7 @@ int hb_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int report, i
             return CMGPU_EINVAL;
         }
     }
+    std::lock_guard<std::mutex> one_call(m->scan_mu);
     HbDev *h = nullptr;
     int rc = hb_prepare(m, &h);
     if (rc) return rc;
@@ -1703,6 +1704,7 @@ int tr_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, const cmgpu_t
             return CMGPU_EINVAL;
         }
     }
+    std::lock_guard<std::mutex> one_call(m->scan_mu);
     HbDev *h = nullptr;
     int rc = hb_prepare(m, &h);
     if (rc) return rc;

@@ -173,6 +173,9 @@ struct cmgpu_model {
     std::vector<float> flog;  // host FLogsum table for null3
     cmx::HbDev *hb = nullptr;  // built on the first HMM-banded scan
     cmx::TrqDev *trq = nullptr;  // built on the first truncated QDB / non-banded scan
+    // held by a HMM-banded or truncated call from its tables to its results:
+    // these calls take no workspace, their buffers belong to the model
+    std::mutex scan_mu;
     // host-only scan plans of the allocation-free entry point (key semiring*8 + qdbidx)
     mutable std::mutex noalloc_mu;
     mutable std::map<int, std::unique_ptr<cmx::Plan>> noalloc_plans;

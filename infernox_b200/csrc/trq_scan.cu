@@ -842,6 +842,7 @@ int trq_batch(const cmgpu_model *mc, cudaStream_t st, int semiring, int qdbidx, 
             return CMGPU_EINVAL;
         }
     }
+    std::lock_guard<std::mutex> one_call(m->scan_mu);
     TrqDev *q = nullptr;
     int rc = trq_prepare(m, &q);
     if (!rc) rc = trq_semiring_tables(m, q, ins);
