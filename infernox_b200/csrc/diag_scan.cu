@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             c.ridx = c.jrel % p.ring_cols;
             const int w0 = g0 + c.w * 32;  // the warp's first column
             c.jmax = w0 < c.ncols ? min(p.W, min(w0 + 32, c.ncols)) : 0;
-            int r = c.j <= wi.jend ? __ldg(dsq + c.j) : 0;
+            int r = c.jrel < c.ncols ? __ldg(dsq + c.j) : 0;  // (j of a later column may wrap)
             r = r > 17 ? 17 : r;
             ring[c.jrel & c.rmask] = (uint8_t)r;
             c.cj = r;
