@@ -63,8 +63,9 @@ struct DiagPlan {
 };
 
 // false when the model is outside the kernel's scope (`why`): another node
-// topology, or (CYK) score tables holding -0, NaN or +inf, for which a
-// floating maximum and the reference's comparison can differ.
+// topology, a single node between ROOT and END, or (CYK) score tables
+// holding -0, NaN or +inf, for which a floating maximum and the reference's
+// comparison can differ.
 bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp, std::string *why);
 
 struct DgParams {

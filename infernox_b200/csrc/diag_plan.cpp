@@ -60,11 +60,18 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
     dp.R = std::max(dp.R, 1);
     // region: ROOT row of local begins, three node buffers (a node's outputs
     // stay until the warp to the right, one phase behind, has read them),
-    // the bifurcations' decks, the saved last columns
+    // the bifurcations' decks, the saved last columns.  A warp begins a group's
+    // first node while the one on its right may be in the group before's ROOT,
+    // which reads buffer (nodes - 2) % 3: where that is the first one, the first
+    // node has a fourth to itself.  (With two nodes ROOT reads that very node.)
     dp.ring_cols = (W + DG_COLS + 31) & ~31;
     int64_t off = (int64_t)(W + 1) * DG_COLS;
     const int64_t buf0 = off;
-    off += 3 * (int64_t)dp.R * DG_ROW;
+    int owners = 0;
+    for (const NodeTopo &t : shape) owners += t.type != END_ND;
+    if (owners < 3) return fail("fewer than three nodes with states of their own");
+    const bool fourth = (owners - 2) % 3 == 0;
+    off += (fourth ? 4 : 3) * (int64_t)dp.R * DG_ROW;
     std::vector<int64_t> deck(nn, 0);
     for (int n = 0; n < nn; n++) {
         const int64_t rows = hi[n] - lo[n] + 1;
@@ -80,7 +87,8 @@ bool build_diag_plan(const cmgpu_cm *cm, const Plan &p, int qdbidx, DiagPlan &dp
     int t = 0;
     for (int n = nn - 1; n >= 0; n--) {
         if (shape[n].type == END_ND) continue;
-        buf[n] = t++ % 3;
+        buf[n] = fourth && t == 0 ? 3 : t % 3;
+        t++;
         DgNode d{};
         d.v0 = shape[n].v0;
         d.type = (int16_t)shape[n].type;

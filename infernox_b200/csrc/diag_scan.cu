@@ -103,7 +103,8 @@ __device__ __forceinline__ void dg_wait(const DgCtx &c, int w, int need) {
 
 // Before a node: the warp on the right has finished the node before the
 // previous one (prev: the step the previous node began with), so it no longer
-// reads the buffer this node writes.
+// reads the buffer this node writes.  (The plan keeps that so from a group's
+// ROOT to the next group's first node.)
 __device__ __forceinline__ void dg_begin_node(DgCtx &c) {
     if (c.w < c.nw - 1) dg_wait(c, c.w + 1, c.prev);
     c.prev = c.step;
@@ -362,15 +363,12 @@ __device__ __forceinline__ void dg_node(const DgParams &p, DgCtx &c, const DgNod
             xl1[y] = ldx(y, d - 1, 1);
         }
     }
-    int ci = 0;  // residue j-d+1
+    int ci = HAS_IL ? c.ring[(c.jrel - d + 1) & c.rmask] : 0;  // residue j-d+1
     for (int r0 = rlo; r0 <= rhi; r0 += DG_CHUNK) {
         const int rend = min(r0 + DG_CHUNK - 1, rhi);
         const int dstop = min(rend, c.jmax);
         const int slot = c.step & (DG_XCH - 1);
         dg_begin_step(c);
-        // after the wait: before a group's first step the warps on the left may
-        // not have written their residues
-        if (HAS_IL) ci = c.ring[(c.jrel - r0 + 1) & c.rmask];
         // the inserts of the column left of the warp: lane r holds span r0 + r
         T hil = ZERO, hir = ZERO;
         if constexpr (HAS_IR) {
@@ -703,10 +701,10 @@ __device__ __forceinline__ void dg_bif(const DgParams &p, DgCtx &c, const DgNode
                 uint32_t *o = out + (int64_t)(d - rlo) * DG_ROW;
                 S::st(o, x);
                 if (need_left) {
-                    // the column left of the group, and the group's last one
-                    // (which takes its place: one warp may hold both)
+                    // the column left of the group, and the group's last one,
+                    // which takes its place (a warp alone holds both)
                     if (c.w == 0 && c.lane == 0) S::st(o - 1, c.first ? fill : S::ld(bnd + (d - rlo) * DG_SLOTS));
-                    __syncwarp();
+                    if (c.nw == 1) __syncwarp();
                     if (!c.last && c.w == c.nw - 1 && c.lane == 31) S::st(bnd + (d - rlo) * DG_SLOTS, x);
                 }
                 if (p.local && beg && in && d >= p.root_dn && d <= p.root_dxcap) {
@@ -779,7 +777,6 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
     if (tid == 0) s_err = 0;
     if (tid < DG_MAX_WARPS) s_prog[tid] = 0;
     c.step = c.prev = 0;
-    c.slack = p.slack;
     if (INS)
         for (int x = tid; x <= p.ilog_nz; x += nthreads) reinterpret_cast<uint16_t *>(dg_smem)[x] = p.ilog[x];
     for (int x = tid; x < p.ring_len; x += nthreads) ring[x] = 0;
@@ -803,13 +800,9 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             const int rows = min(p.nodes[n].rhi, c.ncols) - p.nodes[n].rlo + 1;
             if (rows > 0) c.gsteps += (rows + DG_CHUNK - 1) / DG_CHUNK;
         }
+        c.slack = min(p.slack, c.gsteps);  // never two groups ahead
         for (int g0 = 0; g0 < c.ncols; g0 += cols) {
-            // The right neighbour has finished the whole group before: the node
-            // buffers start again with the first one, which in a third of the
-            // models is the one ROOT still reads its child from (and a group of
-            // fewer steps than the slack would let a warp run two ahead).  About
-            // a step of waiting per group of a thousand.
-            if (c.w < c.nw - 1) dg_wait(c, c.w + 1, c.step + p.stall);
+            if (p.stall && c.w < c.nw - 1) dg_wait(c, c.w + 1, c.step + p.stall);
             c.first = g0 == 0;
             c.last = g0 + cols >= c.ncols;
             c.jrel = g0 + c.col;
@@ -825,7 +818,10 @@ __global__ void __launch_bounds__(32 * DG_MAX_WARPS, 1) diag_kernel(const __grid
             if (p.local && c.jmax > 0)
                 for (int d = p.root_dn; d <= min(p.root_dxcap, c.jmax); d++)
                     S::st(c.reg + c.col + (int64_t)d * DG_COLS, NONE);
-            __syncwarp();  // the first node's fetch copies the begin row of every lane
+            // Before the first node, not only its first step: the node starts with
+            // residues the warps on the left have written for this group, and
+            // copies the begin row of every lane.
+            dg_begin_step(c);
             for (int n = 0; n < p.nnodes; n++) {
                 const DgNode *np = p.nodes + n;
                 dg_begin_node(c);
