@@ -137,16 +137,20 @@ typedef struct cmgpu_stats {
     int32_t kernel;       /* CMGPU_KERNEL_LEVEL, _SWEEP or _DIAG            */
 } cmgpu_stats;
 
-/* Scan kernels of the QDB scanner (cmgpu_workspace_set_kernel).  Both give
+/* Scan kernels of the QDB scanner (cmgpu_workspace_set_kernel).  All give
  * the same results.  LEVEL: one CTA scans up to 16 work items side by side,
  * state by state in dependency levels with CTA barriers (qdb_scan.cu).
  * SWEEP: one warp scans one work item node by node with no CTA barrier
  * (sweep_scan.cu); it needs W <= 255 and the node-local state topology of
- * CMs built by cmbuild.  AUTO picks LEVEL. */
+ * CMs built by cmbuild.  DIAG: one CTA scans one work item, its lanes on
+ * columns (diag_scan.cu); it needs that topology with two nodes or more
+ * between ROOT and END, (CYK) score tables without NaN, +inf and -0, and
+ * device memory for a region per CTA.  AUTO is DIAG where it applies, else
+ * LEVEL. */
 #define CMGPU_KERNEL_AUTO 0
 #define CMGPU_KERNEL_LEVEL 1
 #define CMGPU_KERNEL_SWEEP 2
-#define CMGPU_KERNEL_DIAG 3 /* what AUTO runs; reported in the statistics only */
+#define CMGPU_KERNEL_DIAG 3 /* reported in the statistics only */
 
 typedef struct cmgpu_model cmgpu_model;
 typedef struct cmgpu_workspace cmgpu_workspace;

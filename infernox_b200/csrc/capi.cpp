@@ -427,7 +427,7 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
 
     // kernel choice
     if (calib && ws->kernel == CMGPU_KERNEL_SWEEP) {
-        set_error("cmcalibrate's scan runs on the level kernel only");
+        set_error("cmcalibrate's scan does not run on the node-sweep kernel");
         return CMGPU_EINVAL;
     }
     if (ws->kernel == CMGPU_KERNEL_SWEEP && !dp->sw_ok) {
@@ -435,9 +435,10 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
         return CMGPU_EINVAL;
     }
     // AUTO takes the diagonal kernel wherever it applies (any model with
-    // cm_from_guide's node layout): faster at every size measured, 2.6 against
-    // 26.8 ms for one 300-column window, 112 against 770 ms for 120 uneven
-    // windows.  The level kernel takes the other models.
+    // cm_from_guide's node layout): faster at every size measured, whole calls
+    // 2.3 against 26.8 ms for one 300-column window, 82 against 769 ms for 120
+    // uneven windows.  The level kernel takes the other models, and scans whose
+    // region the device has no memory for.
     const bool diag = dp->dg_ok && ws->kernel == CMGPU_KERNEL_AUTO && !level;
     const bool sweep = dp->sw_ok && ws->kernel == CMGPU_KERNEL_SWEEP;
     const size_t SMEM_CAP = 227 * 1024 - 1024, SM_CAP = 228 * 1024;
@@ -1277,7 +1278,7 @@ int cmgpu_calibrate_scan_batch(const cmgpu_model *m, cmgpu_workspace *ws, int se
                                int do_null3, cmgpu_batch_hit *hits, int32_t cap, int32_t *n_out) {
     if (!dsq_all) return CMGPU_EINVAL;
     if (ws && ws->kernel == CMGPU_KERNEL_SWEEP) {
-        set_error("cmcalibrate's scan runs on the level kernel only");
+        set_error("cmcalibrate's scan does not run on the node-sweep kernel");
         return CMGPU_EINVAL;
     }
     return batch_common(m, ws, semiring, qdbidx, dsq_all, nullptr, dsq_len, wins, nwin, -INFINITY, do_null3, false,

@@ -22,8 +22,10 @@
 //             not matter);
 //   boundary  the last column of every node is saved for the first column of
 //             the next group, so groups repeat no work.
-// All of it is in a per-CTA region of global memory whose working set (two
-// node buffers, about 0.6 MB at W = 148) stays in L2.
+// All of it is in a per-CTA region of global memory.  A CTA works on two node
+// buffers at a time, 0.6 MB each for a MATP node at W = 148, so the 296 CTAs of
+// a full GPU hold more than the L2 does: 39% of the sectors hit, and a cell
+// moves 7.75 bytes of DRAM.
 //
 // Warps run skewed.  A step is one node over 16 spans; a warp starts a step
 // when the warp on its left has finished it, so the column left of its first
@@ -40,10 +42,10 @@
 // cells stay in bounds.
 //
 // Measured on one B200 (before: the level kernel of qdb_scan.cu): Inside,
-// non-banded, M = 379, W = 148, 296 windows of 512: 220 Gcells/s, CYK 335; two
-// 1 kb windows of a 4,629-state model, CYK: 1,809 -> 53 ms.  Bound: the
-// latency of the log-sum chains (LDS and dependent ALU) at 16 warps per SM,
-// 53% of issue slots; DRAM 21%.
+// non-banded, M = 379, W = 148, 296 windows of 512: 219 Gcells/s, CYK 335; two
+// 1 kb windows of a 4,629-state model, CYK, whole call: 1,745 -> 51 ms.  Bound:
+// the latency of the log-sum chains (LDS and dependent ALU) at 16 warps per SM,
+// half of the issue slots; DRAM 26% of the copy bandwidth.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <type_traits>

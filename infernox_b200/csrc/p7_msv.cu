@@ -27,11 +27,13 @@
 //    threshold becomes a candidate (row, xE, leftmost argmax).  A reset only
 //    lowers later rows (the recurrence is monotone and the reset state is the
 //    floor), so the reference's triggers are a subset of the candidates.
-//  * SSV replay: one warp per chunk walks the candidates in row order with
-//    the reference's sequential logic: a candidate at least M-1 rows past the
-//    last reset (or before any reset) is a trigger as it stands; nearer ones
-//    are recomputed from the reset; a trigger is traced back and extended by
-//    lane 0 (the reference's diagonal recovery) and the scan skips past it.
+//  * SSV replay: a warp per segment walks the candidates in row order with
+//    the reference's sequential logic, from the first one that no earlier
+//    trigger can reach to the first such one of a later segment: a candidate
+//    at least M-1 rows past the last reset (or before any reset) is a trigger
+//    as it stands; nearer ones are recomputed from the reset; a trigger is
+//    traced back and extended by lane 0 (the reference's diagonal recovery)
+//    and the scan skips past it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
