@@ -427,7 +427,7 @@ static int scan_windows(cmgpu_model *m, cmgpu_workspace *ws, int semiring, int q
 
     // kernel choice
     if (calib && ws->kernel == CMGPU_KERNEL_SWEEP) {
-        set_error("cmcalibrate's scan does not run on the node-sweep kernel");
+        set_error("cmcalibrate's scan runs on the diagonal or the level kernel only");
         return CMGPU_EINVAL;
     }
     if (ws->kernel == CMGPU_KERNEL_SWEEP && !dp->sw_ok) {
@@ -1278,7 +1278,7 @@ int cmgpu_calibrate_scan_batch(const cmgpu_model *m, cmgpu_workspace *ws, int se
                                int do_null3, cmgpu_batch_hit *hits, int32_t cap, int32_t *n_out) {
     if (!dsq_all) return CMGPU_EINVAL;
     if (ws && ws->kernel == CMGPU_KERNEL_SWEEP) {
-        set_error("cmcalibrate's scan does not run on the node-sweep kernel");
+        set_error("cmcalibrate's scan runs on the diagonal or the level kernel only");
         return CMGPU_EINVAL;
     }
     return batch_common(m, ws, semiring, qdbidx, dsq_all, nullptr, dsq_len, wins, nwin, -INFINITY, do_null3, false,
